@@ -1,5 +1,6 @@
 // Slab sources, DFT monitors and the device step counter.
 
+#include "dft.cuh"
 #include "kernels.cuh"
 
 namespace fdtd {
@@ -39,7 +40,6 @@ __global__ void copy3d_kernel(const float* src, int64_t sr, int64_t sp, float* d
 // window are evaluated once per block into shared memory.
 // beamz/simulation/observe.py:327-357 (gate, window, scale) and 529-585.
 constexpr int kDftThreads = 256;
-constexpr int kDftMaxFreqs = 64;
 
 // Interpolated sample of one (monitor, component, point).  Neighbour-major
 // plan: consecutive points of one neighbour slot are contiguous, and per point
@@ -151,8 +151,6 @@ __global__ void __launch_bounds__(kDftThreads) dft_kernel(DftDev d, const int* c
 // order, with the same gate, window, scale and phase per step as dft_kernel,
 // so the arena is bit-identical to per-step accumulation while it is read
 // and written once per batch.
-constexpr int kDftMaxBatch = 16;
-
 // 128-thread blocks at 32 registers: one fits on an SM beside five resident
 // step CTAs, so sampling on a side stream overlaps the next step.
 constexpr int kDftSampleThreads = 128;
@@ -209,100 +207,10 @@ __global__ void __launch_bounds__(kDftSampleThreads, 16) dft_sample_kernel(DftDe
 
 __global__ void __launch_bounds__(kDftThreads) dft_flush_kernel(DftDev d, const float* samples, const int* counter,
                                                                 int first, int count) {
-  const int mc = blockIdx.y;
-  const int m = mc / 6, c = mc % 6;
-  const int* cnt = d.counts + 5 * m;
-  const int nf = min(max(cnt[0], 0), d.max_freqs);
-  const int np = min(max(cnt[1], 0), d.max_points);
-  const int interval = cnt[2] > 0 ? cnt[2] : 1;
-  const int voff = cnt[3], woff = cnt[4];
-  const float t0 = d.windows[3 * m], t1 = d.windows[3 * m + 1], unit = d.windows[3 * m + 2];
-  __shared__ float s_cos[kDftMaxBatch][kDftMaxFreqs];
-  __shared__ float s_sin[kDftMaxBatch][kDftMaxFreqs];
-  __shared__ float s_scale[kDftMaxBatch];
-  __shared__ float s_window[kDftMaxBatch];
-  __shared__ float s_time[kDftMaxBatch];
-  __shared__ int s_on[kDftMaxBatch];
-  for (int s = threadIdx.x; s < count; s += blockDim.x) {
-    const int step = counter[0] + first + s;
-    int ti = step < 0 ? 0 : step;
-    ti = ti >= d.step_time_len ? d.step_time_len - 1 : ti;
-    const float t = d.step_time[ti];
-    const bool on = step % interval == 0 && t >= t0 && t <= t1;
-    float window = 1.0f;
-    if (on && d.codes[2 * m] == 1 && isfinite(t1) && t1 > t0) {
-      const float span = fmaxf(t1 - t0, 1e-30f);
-      const float tau = fminf(fmaxf((t - t0) / span, 0.0f), 1.0f);
-      window = 0.5f * (1.0f - cosf(6.2831855f * tau));
-    }
-    float scale = fmaxf(window, 0.0f);
-    if (d.codes[2 * m + 1] == 1) {
-      const float phys = ((d.dt * static_cast<float>(interval)) * 299792458.0f) / unit;
-      scale = scale * (phys / sqrtf(6.2831855f));
-    }
-    s_on[s] = on ? 1 : 0;
-    s_scale[s] = scale;
-    s_window[s] = window;
-    s_time[s] = t;
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < count * nf; e += blockDim.x) {
-    const int s = e / nf, f = e % nf;
-    const float theta = (6.2831855f * d.freqs[m * d.max_freqs + f]) * s_time[s];
-    float sn, cs;
-    sincosf(theta, &sn, &cs);
-    s_cos[s][f] = cs;
-    s_sin[s][f] = sn;
-  }
-  __syncthreads();
-  if (c == 0 && blockIdx.x == 0) {
-    for (int f = threadIdx.x; f < nf; f += blockDim.x) {
-      if (woff < 0 || woff + f >= d.weight_len) continue;
-      float ws = d.weight_sum[woff + f];
-      for (int s = 0; s < count; ++s)
-        if (s_on[s]) ws += s_window[s];
-      d.weight_sum[woff + f] = ws;
-    }
-  }
-  const float mask = d.masks[m * 6 + c];
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= np || mask == 0.0f) return;
-  if (voff < 0 || voff + static_cast<int64_t>(6) * nf * np > d.arena_len) return;
-  const int64_t out = voff + (static_cast<int64_t>(c) * nf) * np + p;
-  const int64_t stride = static_cast<int64_t>(d.monitor_count) * 6 * d.max_points;
-  const float* v = samples + (static_cast<int64_t>(m) * 6 + c) * d.max_points + p;
-  // The point's buffered samples are loaded once, and the arena words of
-  // kFlushFreqs frequencies together, so a flush costs a few memory round
-  // trips per point; each arena word still adds the steps in step order.
-  constexpr int kFlushFreqs = 4;
-  float vs[kDftMaxBatch];
-#pragma unroll
-  for (int s = 0; s < kDftMaxBatch; ++s) vs[s] = s < count && s_on[s] ? v[s * stride] : 0.0f;
-  for (int f0 = 0; f0 < nf; f0 += kFlushFreqs) {
-    float re[kFlushFreqs], im[kFlushFreqs];
-#pragma unroll
-    for (int q = 0; q < kFlushFreqs; ++q) {
-      const int64_t o = out + static_cast<int64_t>(f0 + q) * np;
-      re[q] = f0 + q < nf ? d.re[o] : 0.0f;
-      im[q] = f0 + q < nf ? d.im[o] : 0.0f;
-    }
-#pragma unroll
-    for (int q = 0; q < kFlushFreqs; ++q) {
-      const int f = f0 + q;
-      if (f >= nf) break;
-#pragma unroll
-      for (int s = 0; s < kDftMaxBatch; ++s) {
-        if (s >= count) break;
-        if (!s_on[s]) continue;
-        const float sm = s_scale[s] * mask;
-        re[q] += sm * (s_cos[s][f] * vs[s]);
-        im[q] += sm * (s_sin[s][f] * vs[s]);
-      }
-      const int64_t o = out + static_cast<int64_t>(f) * np;
-      d.re[o] = re[q];
-      d.im[o] = im[q];
-    }
-  }
+  __shared__ FlushShared sh;
+  const int m = blockIdx.y / 6, c = blockIdx.y % 6;
+  dft_flush_body<false>(d, sh, samples, counter, first, 0, count, m, c, blockIdx.x * blockDim.x,
+                        c == 0 && blockIdx.x == 0, threadIdx.x, blockDim.x);
 }
 
 __global__ void counter_kernel(int* counter, int nsteps) { counter[0] += nsteps; }

@@ -208,6 +208,10 @@ struct RecorderDev {
   int64_t start[7] = {0, 0, 0, 0, 0, 0, 0};  // prefix sums of the value counts
   float sign[6] = {1, 1, 1, 1, 1, 1};
   int slots[6] = {0, 0, 0, 0, 0, 0};          // gather slots K; 0 = whole component
+  int comp[6] = {0, 0, 0, 0, 0, 0};           // component index
+  struct Box {                                // 2D: the plan is this box of cells, row by row, weight 1
+    int y0 = 0, x0 = 0, ny = 0, nx = 0;       // ny = 0: it is not
+  } box[6];
   const int* idx[6] = {};
   const float* w[6] = {};
   float* values[6] = {};
@@ -222,6 +226,27 @@ struct RecorderDev {
   int step_time_len = 0;
 };
 cudaError_t launch_record(cudaStream_t s, const RecorderDev& r, const int* counter, int step_offset);
+
+// One call's steps of a 2D program (block2d.cu).  `bank[b]` is the step that
+// reads field bank b; `samples` a raw sample ring of `batch` steps
+// ([batch, M, 6, K, P]) or null without monitors.  Sets *done when the steps
+// were enqueued (the recorder counts and the step counter included), else
+// nothing was.
+struct Run2D {
+  int pol = 0;
+  int nsteps = 0, steps_per_launch = 0;
+  Step3D bank[2];
+  int* counter = nullptr;
+  DftDev dft{};
+  float* samples = nullptr;
+  int batch = 0;
+  int nsrc = 0;
+  SourceDev src[kMaxFusedSources];
+  int timing[kMaxFusedSources];
+  int nrec = 0;
+  RecorderDev rec[FDTD_MAX_RECORDERS];
+};
+cudaError_t run_block2d(cudaStream_t s, const Run2D& run, bool* done);
 
 // Gather-plan packing (planner.cu): one (monitor, component) plan.
 struct GatherPackDev {

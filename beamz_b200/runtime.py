@@ -425,6 +425,22 @@ def _pack_plan(lib, stream, indices, weights, dims, strides, device):
     return out_i, out_w
 
 
+def _unit_box(indices, weights, row: int):
+    """(y0, x0, ny, nx) of a one-slot, unit-weight plan that lists a box of a
+    2D component (rows of ``row`` cells) row by row, else four zeros."""
+    i = np.asarray(indices).reshape(len(indices), -1).astype(np.int64)
+    if i.size == 0 or i.shape[1] != 1 or not np.all(np.asarray(weights) == 1):
+        return 0, 0, 0, 0
+    i = i[:, 0]
+    nx = int(np.argmax(np.diff(i) != 1)) + 1 if i.size > 1 and np.any(np.diff(i) != 1) else i.size
+    y0, x0 = divmod(int(i[0]), int(row))
+    if i[0] < 0 or i.size % nx or x0 + nx > row:
+        return 0, 0, 0, 0
+    ny = i.size // nx
+    box = (y0 + np.arange(ny))[:, None] * int(row) + x0 + np.arange(nx)[None, :]
+    return (y0, x0, ny, nx) if np.array_equal(box.reshape(-1), i) else (0, 0, 0, 0)
+
+
 class DeviceProgram:
     """A compiled program: every static input of the step, resident on the device."""
 
@@ -691,6 +707,8 @@ class DeviceProgram:
                 pi, pw = _pack_plan(self.lib, stream, rec.indices[q], rec.weights[q], self.shapes[c],
                                     self._strides(ci), dev)
                 d.indices[q], d.weights[q] = buf(pi), buf(pw)
+                if spec.ndim == 2:
+                    d.box[q][:] = _unit_box(rec.indices[q], rec.weights[q], self.shapes[c][-1])
                 counts.append(int(pi.shape[1]))
             self.recorders.append(counts)
         self._times_for(max(int(spec.total_steps), 1))
@@ -768,6 +786,8 @@ class DeviceProgram:
         for t, term in enumerate(self.e_terms):
             if term.width:
                 s.e_terms[t].psi = abi.buffer_of(state.psi_e[t])
+                if state.psi_e_alt is not None:
+                    s.e_terms[t].psi_alt = abi.buffer_of(state.psi_e_alt[t])
         if self.arena is not None:
             s.dft.re = abi.buffer_of(state.dft_re)
             s.dft.im = abi.buffer_of(state.dft_im)
@@ -823,6 +843,9 @@ class DeviceState:
         self.psi_h = psi_list(program.h_terms, psi_h)
         self.psi_e = psi_list(program.e_terms, psi_e)
         self.psi_h_alt = [torch.empty_like(p) for p in self.psi_h] if fused else None
+        # 2D programs advance several steps per launch, which double-banks the
+        # E-term memories too.
+        self.psi_e_alt = [torch.empty_like(p) for p in self.psi_e] if fused and program.ndim == 2 else None
         a = program.arena
         nv = a.value_count if a else 0
         nw = a.weight_count if a else 0
@@ -831,8 +854,11 @@ class DeviceState:
         self.dft_w = torch.zeros(nw, dtype=torch.float32, device=dev)
         self.dft_samples = None
         if a is not None and program.dft_batch > 1:
-            M, P = len(a.layout), int(a.indices.shape[3])
-            self.dft_samples = torch.empty((program.dft_batch, M, 6, P), dtype=torch.float32, device=dev)
+            # Per buffered step: the interpolated samples, or in 2D every
+            # gather slot's field value (FdtdDft.samples).
+            M, _six, K, P = (int(v) for v in a.indices.shape)
+            shape = (M, 6, K * P) if program.ndim == 2 else (M, 6, P)
+            self.dft_samples = torch.empty((program.dft_batch, *shape), dtype=torch.float32, device=dev)
         self.records = []
         for rec, counts in zip(program.spec.recorders, program.recorders):
             cap = max(0, int(rec.capacity))
@@ -851,6 +877,8 @@ class DeviceState:
         self.fields, self.alt = self.alt, self.fields
         if self.psi_h_alt is not None:
             self.psi_h, self.psi_h_alt = self.psi_h_alt, self.psi_h
+        if self.psi_e_alt is not None:
+            self.psi_e, self.psi_e_alt = self.psi_e_alt, self.psi_e
 
     def set_fields(self, fields: dict) -> None:
         """Load host or device arrays (beamz component shapes) into the current bank."""

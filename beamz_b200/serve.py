@@ -75,11 +75,14 @@ def estimate_bytes(spec: ProgramSpec, schedule: str = "fused") -> int:
         field_bytes = sum(int(np.prod(shapes[c])) * 4 for c in active)
         material = sum(int(np.prod(shapes[c])) * 8 for c in active if c.startswith("E"))
     psi = sum(int(np.prod(t.psi_shape(shapes[t.component]))) * 4 * banks for t in spec.h_terms)
-    psi += sum(int(np.prod(t.psi_shape(shapes[t.component]))) * 4 for t in spec.e_terms)
+    e_banks = banks if spec.ndim == 2 else 1  # 2D programs double-bank the E memories too
+    psi += sum(int(np.prod(t.psi_shape(shapes[t.component]))) * 4 * e_banks for t in spec.e_terms)
     dft = 0
     for m in spec.monitors:
         points = max(int(np.asarray(ix).shape[0]) for ix in m.indices)
-        dft += 6 * len(m.freqs) * points * 8 * 2 + 6 * points * 8 * 8 + 16 * 6 * points * 4  # + sample batch
+        slots = max(np.asarray(ix).size // max(1, len(ix)) for ix in m.indices)
+        per = slots if spec.ndim == 2 else 1  # sample batch: every slot's value in 2D
+        dft += 6 * len(m.freqs) * points * 8 * 2 + 6 * points * 8 * 8 + 16 * 6 * points * 4 * per
     records = 0
     for r in spec.recorders:
         for q, c in enumerate(r.components):

@@ -24,7 +24,7 @@ extern "C" {
 #endif
 
 /* Bumped whenever a struct below changes layout (beamz: abi_layout.json "abi_version"). */
-#define FDTD_ABI_VERSION 13
+#define FDTD_ABI_VERSION 14
 
 /* Element types (beamz: cuda/src/launch.h:6-10, plus U8 for voxel ids and F64
  * for reduction results). */
@@ -128,7 +128,10 @@ typedef struct FdtdBuffer {
  * beamz/simulation/kernels.py:238-264).  a/b/inv_kappa are 1-D of length
  * low + high along `axis` (0 = z, 1 = y, 2 = x of the target component);
  * psi has the target component's shape with that axis replaced by low + high.
- * psi_alt is the second psi bank used by FDTD_SCHEDULE_FUSED for H terms. */
+ * psi_alt is the second psi bank used by FDTD_SCHEDULE_FUSED for H terms; a 2D
+ * program may carry one for every nonempty E term too, which then alternates
+ * like the H terms' (an odd step count leaves the result in psi_alt) and lets
+ * fdtd_launch_program advance several steps per launch. */
 typedef struct FdtdCpmlTerm {
   int32_t axis;
   int32_t low;
@@ -164,7 +167,8 @@ typedef struct FdtdSource {
  *  windows  F32 [M, 3]: t_start, t_end, length_unit
  *  re, im   F32 arena, accumulated at value_offset + (c * F + f) * P + p
  *  weight_sum F32 arena, accumulated at weight_offset + f
- *  samples  F32 [batch, M, 6, P] (optional step batching)                      */
+ *  samples  F32 [batch, M, 6, P] (optional step batching); 2D programs may pass
+ *           [batch, M, 6, K, P], room for every gather slot's value             */
 typedef struct FdtdDft {
   int32_t monitor_count;
   int32_t batch;           /* > 1 with `samples`: accumulate every `batch` steps (below) */
@@ -222,6 +226,10 @@ typedef struct FdtdRecorder {
   FdtdBuffer steps;         /* S32 [capacity] */
   FdtdBuffer times;         /* F32 [capacity] */
   FdtdBuffer count;         /* S32 [2] */
+  /* 2D programs, optional: value set q's plan, when it is a box of cells with
+   * unit weights in row order, as (y0, x0, ny, nx); ny = 0: it is not.  The
+   * indices and weights still describe it. */
+  int32_t box[6][4];
 } FdtdRecorder;
 
 /* A complete step program (replaces BeamzLaunch + BeamzProgramLaunch,
