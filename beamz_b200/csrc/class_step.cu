@@ -563,15 +563,23 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
   for (int e = tid; e < 256; e += T::NT) sm.cls[e] = p.class_coef[e];
   if constexpr (Lossy)
     for (int e = tid; e < 64 * 4; e += T::NT) sm.hcls[e] = p.h_class_coef[e];
+  // CPML coefficient slabs, one (term, slot) per thread and round, so that every
+  // load of the table is in flight together.  Term by term, the twelve dependent
+  // round trips held up a CTA's first plane (us per step: 512 x 512 x 256 929
+  // -> 919, 192^3 249 -> 244, 277 x 203 x 150 275 -> 268).
   bool cc_smem = true;
   if (Cpml) {
 #pragma unroll
     for (int t = 0; t < 12; ++t) {
       const CpmlTermDev& d = t < 6 ? p.ht[t] : p.et[t - 6];
-      const int w = d.low + d.high;
-      cc_smem = cc_smem && w <= kSlots;
-      for (int e = tid; e < w && e < kSlots; e += T::NT)
-        sm.cc[t][e] = make_float4(Exact ? d.a[e] : d.a[e] * inv_res, d.b[e], d.k[e], 0.0f);
+      cc_smem = cc_smem && d.low + d.high <= kSlots;
+    }
+#pragma unroll
+    for (int e = tid; e < 12 * kSlots; e += T::NT) {
+      const int t = e / kSlots, slot = e % kSlots;
+      const CpmlTermDev& d = t < 6 ? p.ht[t] : p.et[t - 6];
+      if (slot < d.low + d.high)
+        sm.cc[t][slot] = make_float4(Exact ? d.a[slot] : d.a[slot] * inv_res, d.b[slot], d.k[slot], 0.0f);
     }
   }
   if (tid < p.n_hsrc) sm.amp[tid] = source_amplitude(p.hsrc[tid], p.step_counter[0] + p.step_offset);
