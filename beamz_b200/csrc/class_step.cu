@@ -34,12 +34,12 @@
 //
 // The tiles end at x = X - 1 (a partial last tile masks its stores past X)
 // and the lattice column x = X is a small column kernel's, run before the
-// step.  Tile-planes that touch a z face or an H source run a general
+// step.  Tile-planes that touch an H source run a general
 // per-cell path with every validity, ghost and PEC rule; the rest run
 // a straight body compiled for their case: the interior, the x = 0 / y = 0
 // faces, the x-slab tiles (about half of them on a 512-wide grid), the other
-// absorber tiles (axes as plane-uniform run-time flags), and the last tile
-// row, shifted down to end at row Y (where Hx, Hz and Ey do not exist and the
+// absorber tiles and the z faces (axes as plane-uniform run-time flags), and
+// the last tile row, shifted down to end at row Y (where Hx, Hz and Ey do not exist and the
 // y = Y ghost applies) with its rows below the tile row before computed but
 // not stored.  The H-term CPML memories are double-banked (the halo
 // recomputation reads them), the E-term ones updated in place.
@@ -723,8 +723,8 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
     const uint8_t* HIDS = sm.hids[Lossy ? hs : 0];  // Lossy: H classes, box column = x - i0 + 16
     const bool src = p.n_hsrc > 0 && sources_touch(p, k, j0 - 1, j0 + TY, i0 - 1, i0 + TX);
 
-    if (fast_ok && !src && k >= 1 && k < Z) {
-      // ---- straight tile-plane: every own and halo cell valid ----------------
+    if (fast_ok && !src) {
+      // ---- straight tile-plane ----------------------------------------------------
       auto body = [&](auto mode) {
         // The body's CPML axes (bits 0-2: x, y, z) and whether the tile may
         // touch x = 0 / y = 0 (bit 3) are compile-time, so that a tile-plane
@@ -744,6 +744,13 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
         const bool lyr = LY || (RT && ylast);
         const bool st = !lyr || own;       // this row is stored
         const bool rowY = lyr && j == Y;   // row Y: Hx, Hz, Ey absent
+        // The same bodies take the z faces: plane 0 (the ghost beyond z = 0) and
+        // plane Z (Hx, Hy and Ez do not exist there -- nothing of theirs, psi
+        // included, is read or written -- and the ghost beyond z = Z applies).
+        // On the general path such a plane took three times an absorber plane's
+        // time (us per step: 512 x 512 x 256 919 -> 909, 256 x 192 x 128
+        // rectilinear 155 -> 147).
+        const bool z0 = (RT || LY) && k == 0, zZ = (RT || LY) && k == Z;
         const bool AX = SX && (!RT || shell_x), AY = SY && (!RT || shell_y), AZ = SZ && (!RT || shell_z);
         const bool at_x0 = FC && xface, at_y0 = FC && yface;
         const int jh = j0 - 1, ih = i0 - 1;  // the halo row and column
@@ -756,10 +763,10 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
         // psi of the H terms: own cells and halos.
         float4 qh0, qh1, qh2, qh5;
         if (AY && !rowY) {
-          qh0 = psi4_fetch<1>(p.ht[0], slot_of(p.ht[0], j), k, j, i, nvv);
+          if (!zZ) qh0 = psi4_fetch<1>(p.ht[0], slot_of(p.ht[0], j), k, j, i, nvv);
           qh5 = psi4_fetch<1>(p.ht[5], slot_of(p.ht[5], j), k, j, i, nvv);
         }
-        if (AZ) {
+        if (AZ && !zZ) {
           if (!rowY) qh1 = psi4_fetch<0>(p.ht[1], slot_of(p.ht[1], k), k, j, i, nvv);
           qh2 = psi4_fetch<0>(p.ht[2], slot_of(p.ht[2], k), k, j, i, nvv);
         }
@@ -768,7 +775,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
         if (emit) {
           if (AY) {
             qe0 = psi4_fetch<1>(p.et[0], slot_of(p.et[0], j), k, j, i, nvv);
-            qe5 = psi4_fetch<1>(p.et[5], slot_of(p.et[5], j), k, j, i, nvv);
+            if (!zZ) qe5 = psi4_fetch<1>(p.et[5], slot_of(p.et[5], j), k, j, i, nvv);
           }
           if (AZ) {
             qe1 = psi4_fetch<0>(p.et[1], slot_of(p.et[1], k), k, j, i, nvv);
@@ -780,7 +787,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int w = sm.xst[4 + h][lane];
-            if ((w & 1) && !(rowY && (w & 2))) {
+            if ((w & 1) && !(rowY && (w & 2)) && !(zZ && !(w & 2))) {
               const bool second = w & 2;  // Hzx (dEy/dx), else Hyx (dEz/dx)
               const int slot = (w >> 2) & 63, xo = w >> 8;
               const CpmlTermDev& d = second ? p.ht[4] : p.ht[3];
@@ -811,10 +818,10 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           dz0 = MH4x(sub4(next4(ey, ey4), ey), i), dz1 = MH4(sub4(ld4(E0x + rc + BX), ex), 1, j);  // Hz: dEy/dx, dEx/dy
         }
         if (AY && !rowY) {
-          dx0 = psi4_apply<Exact, 1>(p.ht[0], sm.cc[0], slot_of(p.ht[0], j), qh0, k, j, i, res, dx0, emit && st, nvv);
+          if (!zZ) dx0 = psi4_apply<Exact, 1>(p.ht[0], sm.cc[0], slot_of(p.ht[0], j), qh0, k, j, i, res, dx0, emit && st, nvv);
           dz1 = psi4_apply<Exact, 1>(p.ht[5], sm.cc[5], slot_of(p.ht[5], j), qh5, k, j, i, res, dz1, emit && st, nvv);
         }
-        if (AZ) {
+        if (AZ && !zZ) {
           if (!rowY)
             dx1 = psi4_apply<Exact, 0>(p.ht[1], sm.cc[1], slot_of(p.ht[1], k), qh1, k, j, i, res, dx1, emit && st, nvv);
           dy0 = psi4_apply<Exact, 0>(p.ht[2], sm.cc[2], slot_of(p.ht[2], k), qh2, k, j, i, res, dy0, emit && st, nvv);
@@ -837,18 +844,19 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
         if (at_x0 && lane == 0 && wx0) hx.x = 0.0f;  // PEC: normal H on the x = 0 wall
         if (at_y0 && warp == 0 && wy0) hy = make_float4(0.f, 0.f, 0.f, 0.f);
         if (rowY && wy1) hy = make_float4(0.f, 0.f, 0.f, 0.f);  // PEC: normal H on the y = Y wall
+        if ((z0 && wz0) || (zZ && wz1)) hz = make_float4(0.f, 0.f, 0.f, 0.f);  // ... on the z walls
         st4(&sm.hn[0][r][c0], hx);
         st4(&sm.hn[1][r][c0], hy);
         st4(&sm.hn[2][r][c0], hz);
         const int o = k * PL + j * P + i;
         if (emit && st) {
-          if (!rowY) st4m(p.hout[0] + o, hx, nvv);
-          st4m(p.hout[1] + o, hy, nvv);
+          if (!rowY && !zZ) st4m(p.hout[0] + o, hx, nvv);
+          if (!zZ) st4m(p.hout[1] + o, hy, nvv);
           if (!rowY) st4m(p.hout[2] + o, hz, nvv);
         }
         // ---- recomputed halo: row j0-1 (Hx by warp 0, Hz by warp 1) and
         //      column i0-1 (Hy, Hz by warp 2), read-only on psi ----
-        if (halo_row_x) {
+        if (halo_row_x && !zZ) {
           const int b = c0;
           float4 qa, qb;
           if (AY) qa = psi4_fetch<1>(p.ht[0], slot_of(p.ht[0], jh), k, jh, i, nvv);
@@ -883,21 +891,24 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           float4 d0 = MH4x(sub4(next4(eyh, e4), eyh), i), d1 = MH4(sub4(ld4(E0x + b + BX), ld4(E0x + b)), 1, jh);
           if (AX) d0 = psix_apply<Exact>(p.ht[4], sm.cc[4], xs4, qa, k, jh, res, d0, false);
           if (AY) d1 = psi4_apply<Exact, 1>(p.ht[5], sm.cc[5], slot_of(p.ht[5], jh), qb, k, jh, i, res, d1, false, nvv);
+          float4 h;
           if constexpr (Lossy)
-            st4(&sm.hn[2][0][b], h4_loss<Exact>(ld4(HOz + b), sm.hcls,
-                                                *reinterpret_cast<const uint32_t*>(HIDS + 16 + 4 * lane), 2, d0, d1));
+            h = h4_loss<Exact>(ld4(HOz + b), sm.hcls, *reinterpret_cast<const uint32_t*>(HIDS + 16 + 4 * lane), 2, d0,
+                               d1);
           else
-            st4(&sm.hn[2][0][b], h4<Exact>(ld4(HOz + b), sm.hcoef[2], sm.hcoef[5], d0, d1));
+            h = h4<Exact>(ld4(HOz + b), sm.hcoef[2], sm.hcoef[5], d0, d1);
+          if ((z0 && wz0) || (zZ && wz1)) h = make_float4(0.f, 0.f, 0.f, 0.f);
+          st4(&sm.hn[2][0][b], h);
         } else if (halo_col) {
           const int rr = 1 + lane, b = rr * BX + 3;
           const bool hz_ok = !(lyr && jc == Y);  // Hz has no row Y
           float qc0 = 0.f, qc1 = 0.f, qc2 = 0.f, qc3 = 0.f;
-          if (AZ) qc0 = psi1_fetch<0>(p.ht[2], k, jc, ih);
-          if (AX) qc1 = psi1_fetch<2>(p.ht[3], k, jc, ih);
+          if (AZ && !zZ) qc0 = psi1_fetch<0>(p.ht[2], k, jc, ih);
+          if (AX && !zZ) qc1 = psi1_fetch<2>(p.ht[3], k, jc, ih);
           if (AX && hz_ok) qc2 = psi1_fetch<2>(p.ht[4], k, jc, ih);
           if (AY && hz_ok) qc3 = psi1_fetch<1>(p.ht[5], k, jc, ih);
           float d0 = MH(E1x[b] - E0x[b], 0, k), d1 = MH(E0z[b + 1] - E0z[b], 2, ih);  // Hy: dEx/dz, dEz/dx
-          if (AZ) d0 = psi1_apply<Exact, 0>(p.ht[2], sm.cc[2], qc0, k, jc, ih, res, d0, false);
+          if (AZ && !zZ) d0 = psi1_apply<Exact, 0>(p.ht[2], sm.cc[2], qc0, k, jc, ih, res, d0, false);
           if (AX) d1 = psi1_apply<Exact, 2>(p.ht[3], sm.cc[3], qc1, k, jc, ih, res, d1, false);
           const int hc = Lossy ? (HIDS[rr * T::HW + 15] & kHClassMask) : 0;  // the halo column's H class
           const float2 cy = Lossy ? sm.hcls[hc * 4 + 1] : make_float2(sm.hcoef[1], sm.hcoef[4]);
@@ -908,7 +919,9 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           if (AX && hz_ok) f0 = psi1_apply<Exact, 2>(p.ht[4], sm.cc[4], qc2, k, jc, ih, res, f0, false);
           if (AY && hz_ok) f1 = psi1_apply<Exact, 1>(p.ht[5], sm.cc[5], qc3, k, jc, ih, res, f1, false);
           sm.hn[1][rr][3] = hyv;
-          sm.hn[2][rr][3] = h1<Exact>(HOz[b], cz.x, cz.y, f0, f1);
+          float hzv = h1<Exact>(HOz[b], cz.x, cz.y, f0, f1);
+          if ((z0 && wz0) || (zZ && wz1)) hzv = 0.0f;
+          sm.hn[2][rr][3] = hzv;
         }
         __syncthreads();
         if (!emit) {
@@ -921,7 +934,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int w = sm.xst[6 + h][lane];
-            if ((w & 1) && !(rowY && !(w & 2))) {
+            if ((w & 1) && !(rowY && !(w & 2)) && !(zZ && (w & 2))) {
               const bool second = w & 2;  // Ezx (dHy/dx), else Eyx (dHz/dx)
               const int slot = (w >> 2) & 63, xo = w >> 8;
               const CpmlTermDev& d = second ? p.et[4] : p.et[3];
@@ -955,8 +968,14 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           hzy = wy0 ? make_float4(0.f, 0.f, 0.f, 0.f) : hz;
           hxy = wy0 ? make_float4(0.f, 0.f, 0.f, 0.f) : hx;
         }
-        float4 fx0 = ME4(sub4(hz, hzy), 1, j), fx1 = ME4(sub4(hy, hyp), 0, k);        // Ex: dHz/dy, dHy/dz
-        float4 fy0 = ME4(sub4(hx, hxp), 0, k), fy1 = ME4x(sub4(hz, prev4(hzl, hz)), i);  // Ey: dHx/dz, dHz/dx
+        float4 ghy = sub4(hy, hyp), ghx = sub4(hx, hxp);  // along z
+        if (z0 || zZ) {  // ghost beyond z = 0 / z = Z: zero on a metallic wall, else the edge value
+          const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+          ghy = z0 ? (wz0 ? hy : z4) : (wz1 ? sub4(z4, hyp) : z4);
+          ghx = z0 ? (wz0 ? hx : z4) : (wz1 ? sub4(z4, hxp) : z4);
+        }
+        float4 fx0 = ME4(sub4(hz, hzy), 1, j), fx1 = ME4(ghy, 0, k);        // Ex: dHz/dy, dHy/dz
+        float4 fy0 = ME4(ghx, 0, k), fy1 = ME4x(sub4(hz, prev4(hzl, hz)), i);  // Ey: dHx/dz, dHz/dx
         float4 fz0 = ME4x(sub4(hy, prev4(hyl, hy)), i), fz1 = ME4(sub4(hx, hxy), 1, j);  // Ez: dHy/dx, dHx/dy
         if (rowY) {  // ghost beyond y = Y: zero on a metallic wall, else the edge value
           const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -965,7 +984,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
         }
         if (AY) {
           fx0 = psi4_apply<Exact, 1>(p.et[0], sm.cc[6], slot_of(p.et[0], j), qe0, k, j, i, res, fx0, st, nvv);
-          fz1 = psi4_apply<Exact, 1>(p.et[5], sm.cc[11], slot_of(p.et[5], j), qe5, k, j, i, res, fz1, st, nvv);
+          if (!zZ) fz1 = psi4_apply<Exact, 1>(p.et[5], sm.cc[11], slot_of(p.et[5], j), qe5, k, j, i, res, fz1, st, nvv);
         }
         if (AZ) {
           fx1 = psi4_apply<Exact, 0>(p.et[1], sm.cc[7], slot_of(p.et[1], k), qe1, k, j, i, res, fx1, st, nvv);
@@ -1006,23 +1025,28 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           nx = make_float4(0.f, 0.f, 0.f, 0.f);
           nz = nx;
         }
+        if ((z0 && wz0) || (zZ && wz1)) {  // Ex, Ey on the z walls
+          nx = make_float4(0.f, 0.f, 0.f, 0.f);
+          ny = nx;
+        }
         if (st) {
           st4m(p.eout[0] + o, nx, nvv);
           if (!rowY) st4m(p.eout[1] + o, ny, nvv);
-          st4m(p.eout[2] + o, nz, nvv);
+          if (!zZ) st4m(p.eout[2] + o, nz, nvv);
         }
         hxp = hx;
         hyp = hy;
       };
       using std::integral_constant;
       if constexpr (!Cpml) {
-        if (ylast || i0 + TX > X) body(integral_constant<int, 32 | 8>{});  // last row, partial last tile
+        if (ylast || i0 + TX > X || k == 0 || k == Z)
+          body(integral_constant<int, 32 | 8>{});  // last row, partial last tile, z faces
         else if (xface || yface) body(integral_constant<int, 8>{});
         else body(integral_constant<int, 0>{});
       } else {
         shell_z = !(k >= p.cpml_inner[0][0] && k < p.cpml_inner[0][1]);
-        if (ylast || shell_y || shell_z || i0 + TX > X)
-          body(integral_constant<int, 16 | 8 | 7>{});  // last row, y / z slabs, partial last tile
+        if (ylast || shell_y || shell_z || i0 + TX > X || k == 0 || k == Z)
+          body(integral_constant<int, 16 | 8 | 7>{});  // last row, y / z slabs, partial last tile, z faces
         else if (shell_x) body(integral_constant<int, 8 | 1>{});           // x slab tiles (about half)
         else if (xface || yface) body(integral_constant<int, 8>{});
         else body(integral_constant<int, 0>{});
