@@ -55,6 +55,7 @@ EXPORTED_SYMBOLS = (
     "fdtd_voxel_histogram",
     "fdtd_monitor_reduce",
     "fdtd_adjoint_step_noalloc",
+    "fdtd_adjoint_steps",
     "fdtd_graph_create",
     "fdtd_graph_launch",
     "fdtd_graph_destroy",
@@ -339,6 +340,9 @@ def load_library(path: str | None = None):
         lib.fdtd_adjoint_step_noalloc.argtypes = [ctypes.c_void_p, ctypes.POINTER(FdtdProgram),
                                                   ctypes.POINTER(FdtdAdjointStep)]
         lib.fdtd_adjoint_step_noalloc.restype = ctypes.c_int
+        lib.fdtd_adjoint_steps.argtypes = [ctypes.c_void_p, ctypes.POINTER(FdtdProgram), ctypes.POINTER(FdtdAdjointStep),
+                                           ctypes.c_int32]
+        lib.fdtd_adjoint_steps.restype = ctypes.c_int
         lib.fdtd_field_diagnostics.argtypes = [ctypes.c_void_p, ctypes.POINTER(FdtdProgram),
                                                ctypes.POINTER(FdtdDiagnostics)]
         lib.fdtd_field_diagnostics.restype = ctypes.c_int

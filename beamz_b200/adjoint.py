@@ -13,7 +13,7 @@ coefficients c = dt / (eps0 eps_site) inside a design box:
   segment by segment from the last: restore the checkpoint and recompute the
   segment's steps while ``fdtd_adjoint_curl`` stores the curl after every
   step (the same differences and divisions, so the same bits).  Then
-  ``fdtd_adjoint_step`` runs for the steps in reverse.  Each adjoint step
+  ``fdtd_adjoint_steps`` runs the steps in reverse.  Each adjoint step
   injects the DFT adjoint source of that step's sample, transposes the E and
   H updates exactly (CPML memories, ghost planes and metallic walls included)
   and accumulates dJ/dc += mu * curl over the box.
@@ -37,10 +37,6 @@ import numpy as np
 
 from . import abi
 from .plan import COMPONENT_INDEX, COMPONENTS, ProgramSpec, active_components, component_shape
-
-# E component each E term differentiates the H of (3D term order), and vice versa.
-_E_TERM_SRC = (5, 4, 3, 5, 4, 3)
-_H_TERM_SRC = (2, 1, 0, 2, 1, 0)
 
 
 def _torch():
@@ -217,15 +213,10 @@ class AdjointProblem:
         return self.dft[0], self.dft[1]
 
     # -- backward -------------------------------------------------------------
-    def _step_struct(self, step: int, scratch_e, scratch_h, g_re, g_im, curls, grads):
+    def _step_struct(self, step: int, g_re, g_im, curls, grads):
         a = abi.FdtdAdjointStep()
         a.abi_version = abi.FDTD_ABI_VERSION
         a.step = int(step)
-        for t in range(6):
-            if scratch_e[t] is not None:
-                a.scratch_e[t] = abi.buffer_of(scratch_e[t])
-            if scratch_h[t] is not None:
-                a.scratch_h[t] = abi.buffer_of(scratch_h[t])
         if g_re is not None:
             a.dft_grad_re = abi.buffer_of(g_re)
             a.dft_grad_im = abi.buffer_of(g_im)
@@ -239,6 +230,13 @@ class AdjointProblem:
         a.box_hi[:] = list(self.box_hi)
         return a
 
+    def _adjoint_steps(self, lam, s0: int, s1: int, g_re, g_im, curls, grads):
+        """The adjoint of steps s1-1 .. s0, ``curls`` their [steps, box] curls."""
+        a = self._step_struct(s1 - 1, g_re, g_im, curls, grads)
+        s = self.adjoint_program.fill(lam, 0)
+        abi.check(self.lib.fdtd_adjoint_steps(self.runtime._stream(self.adjoint_program), ctypes.byref(s),
+                                              ctypes.byref(a), s1 - s0), "fdtd_adjoint_steps")
+
     def backward(self, g_re=None, g_im=None):
         """dJ/dc per active E component (beamz shapes; zero outside the box)
         for dJ/d(dft re) = g_re and dJ/d(dft im) = g_im."""
@@ -247,56 +245,35 @@ class AdjointProblem:
         dev = self.device
         if self.dft is None:
             raise RuntimeError("run forward() first")
-        shapes = self.adjoint_program.shapes
         lam = rt.initial_state(self.adjoint_program)  # adjoint fields and memories, zero
-        prog = self.adjoint_program
-        scratch_e = [None] * 6
-        scratch_h = [None] * 6
-        for t in range(6):
-            ec, hs = COMPONENTS[t // 2], COMPONENTS[_E_TERM_SRC[t]]
-            if ec in self.active and hs in self.active:
-                scratch_e[t] = torch.zeros(shapes[ec], dtype=torch.float32, device=dev)
-            hc, es = COMPONENTS[3 + t // 2], COMPONENTS[_H_TERM_SRC[t]]
-            if hc in self.active and es in self.active:
-                scratch_h[t] = torch.zeros(shapes[hc], dtype=torch.float32, device=dev)
         if g_re is not None or g_im is not None:
             g_re = torch.zeros_like(self.dft[0]) if g_re is None else g_re.detach().float().contiguous()
             g_im = torch.zeros_like(self.dft[1]) if g_im is None else g_im.detach().float().contiguous()
         grads = [None] * 3
         for c in self.e_active:
             grads[COMPONENT_INDEX[c]] = torch.zeros(self.box_shape, dtype=torch.float32, device=dev)
-        stream = rt._stream(prog)
         if self.curl_record is not None:  # curls from the forward's recorded H, 256 steps at a time
             for s1 in range(self.nsteps, 0, -256):
                 s0 = max(0, s1 - 256)
-                curl_all = self._curls(self._state, s0, s1)
-                for n in reversed(range(s0, s1)):
-                    curls = [None if c is None else c[n - s0] for c in curl_all]
-                    a = self._step_struct(n, scratch_e, scratch_h, g_re, g_im, curls, grads)
-                    s = prog.fill(lam, 0)
-                    abi.check(self.lib.fdtd_adjoint_step(stream, ctypes.byref(s), ctypes.byref(a)),
-                              "fdtd_adjoint_step")
-                del curl_all
+                self._adjoint_steps(lam, s0, s1, g_re, g_im, self._curls(self._state, s0, s1), grads)
             return self._finish(lam, grads)
         fprog = self.forward_program
+        stream = rt._stream(fprog)
         rstate = rt.initial_state(fprog)
         nseg = len(self.checkpoints)
         for seg in reversed(range(nseg)):
             s0 = seg * self.every
             s1 = min(s0 + self.every, self.nsteps)
             self._restore(rstate, self.checkpoints[seg])
-            curls = [[None] * 3 for _ in range(s1 - s0)]
+            curls = [None] * 3
+            for c in self.e_active:
+                curls[COMPONENT_INDEX[c]] = torch.empty((s1 - s0, *self.box_shape), dtype=torch.float32, device=dev)
             for n in range(s0, s1):
                 rt.run_steps(rstate, fprog, 1)
-                for c in self.e_active:
-                    curls[n - s0][COMPONENT_INDEX[c]] = torch.empty(self.box_shape, dtype=torch.float32, device=dev)
-                a = self._step_struct(n, [None] * 6, [None] * 6, None, None, curls[n - s0], None)
+                a = self._step_struct(n, None, None, [None if c is None else c[n - s0] for c in curls], None)
                 s = fprog.fill(rstate, 0)
                 abi.check(self.lib.fdtd_adjoint_curl(stream, ctypes.byref(s), ctypes.byref(a)), "fdtd_adjoint_curl")
-            for n in reversed(range(s0, s1)):
-                a = self._step_struct(n, scratch_e, scratch_h, g_re, g_im, curls[n - s0], grads)
-                s = prog.fill(lam, 0)
-                abi.check(self.lib.fdtd_adjoint_step(stream, ctypes.byref(s), ctypes.byref(a)), "fdtd_adjoint_step")
+            self._adjoint_steps(lam, s0, s1, g_re, g_im, curls, grads)
             del curls
         rstate.check()
         return self._finish(lam, grads)

@@ -26,12 +26,16 @@
 //   difference carries its coordinate's inverse distance instead of 1/res:
 //   (D^T u)[m] = mh[m-1] u[m-1] - mh[m] u[m] and
 //   (B^T t)[h] = r(h) me[h] t[h] - r(h+1) me[h+1] t[h+1].
-// Each transpose is split into a per-target pass that writes lam_d into a
-// scratch array (one per derivative term) and a per-source gather, so no
-// two threads write one element.  The permittivity gradient accumulates
-// mu * curl'_n per E site over a design box, mu = the masked E adjoint and
-// curl'_n the forward curl recomputed from a checkpoint.
-
+// Every lambda_d is recomputed where it is gathered, from the adjoint fields,
+// the coefficients and the memories of its site (a handful of L1 / L2 hits),
+// instead of travelling through one scratch array per term: a step is three
+// kernels.  The H pass reads the E adjoint fields, the E pass the new H ones,
+// each writing only its own sites, and each set of memories is updated when its
+// last reader is done (psi_E by the E pass, psi_H by the third kernel, over the
+// absorber slabs alone).  With scratch and one launch per component and pass, a
+// 256 x 256 x 128 step moved 1.7 GB in twelve launches; this form 0.7 GB.  The
+// permittivity gradient accumulates mu * curl'_n per E site over a design box,
+// mu = the masked E adjoint and curl'_n the forward curl.
 
 #include "kernels.cuh"
 
@@ -50,159 +54,202 @@ __host__ __device__ constexpr int adj_axis(int t) { return (t == 0 || t == 5) ? 
 
 constexpr int kAdjThreads = 256;
 
-// Element offsets of a component fit 32 bits (every entry point validates
-// arrays below 2^31 elements), so the split is two 32-bit divisions rather
-// than 64-bit ones, which the GPU emulates in dozens of instructions.
-__device__ __forceinline__ void unflat(int64_t idx, const Dims& d, int& k, int& j, int& i) {
-  const unsigned id = static_cast<unsigned>(idx), dx = static_cast<unsigned>(d.x), dy = static_cast<unsigned>(d.y);
-  const unsigned r = id / dx;
-  i = static_cast<int>(id - r * dx);
-  k = static_cast<int>(r / dy);
-  j = static_cast<int>(r - static_cast<unsigned>(k) * dy);
-}
+// Element offsets fit 32 bits (every entry point validates arrays below 2^31
+// elements).
+__device__ __forceinline__ int at(const Dims& d, int k, int j, int i) { return (k * d.y + j) * d.x + i; }
 
 __device__ __forceinline__ int coord_of(int axis, int k, int j, int i) { return axis == 0 ? k : (axis == 1 ? j : i); }
 
-__device__ __forceinline__ int64_t psi_index(const CpmlTermDev& t, int axis, int slot, int k, int j, int i) {
+__device__ __forceinline__ int psi_index(const CpmlTermDev& t, int axis, int slot, int k, int j, int i) {
   const int pk = axis == 0 ? slot : k, pj = axis == 1 ? slot : j, pi = axis == 2 ? slot : i;
-  return (static_cast<int64_t>(pk) * t.pdy + pj) * static_cast<int64_t>(t.pdx) + pi;
+  return (pk * t.pdy + pj) * t.pdx + pi;
 }
 
-// Transpose of one CPML-corrected derivative at a site: lam_d' -> lam_d,
-// updating the adjoint memory (held in psi_out) in place.
+__device__ __forceinline__ float coef_at(const float* p, int full, int idx) { return p[full ? idx : 0]; }
+
+// Transpose of one CPML-corrected derivative at a site: lam_d' -> lam_d from the
+// adjoint memory (held in psi_out), which stays as it is (Update: advances).
+template <bool Update>
 __device__ __forceinline__ float cpml_transpose(const CpmlTermDev& t, int axis, int k, int j, int i, float ld) {
   const int slot = cpml_slot(t, coord_of(axis, k, j, i));
   if (slot < 0) return ld;
-  const int64_t off = psi_index(t, axis, slot, k, j, i);
+  const int off = psi_index(t, axis, slot, k, j, i);
   const float acc = t.psi_out[off] + ld;
-  t.psi_out[off] = t.b[slot] * acc;
+  if (Update) t.psi_out[off] = t.b[slot] * acc;
   return t.k[slot] * ld + t.a[slot] * acc;
 }
 
-__device__ __forceinline__ float coef_at(const float* p, int full, int64_t idx) { return p[full ? idx : 0]; }
-
-// 4a. E transpose, per E site of component c: mask, identity part, the two
-// terms' lam_d into scratch, and the design-box gradient.
-template <int c>
-__global__ void __launch_bounds__(kAdjThreads) adj_e_kernel(Step3D p, AdjDev a) {
+// lam_d of E term t at its E site, from the E adjoint field before the E pass.
+__device__ __forceinline__ float e_term(const Step3D& p, const AdjDev& a, int t, int k, int j, int i) {
+  const int c = t / 2;
   const Dims d = component_dims(c, p.Z, p.Y, p.X);
-  const int64_t n = static_cast<int64_t>(d.z) * d.y * d.x;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < n;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int k, j, i;
-    unflat(idx, d, k, j, i);
-    float mu = a.lam[c][idx];
-    if (e_constrained(p.metallic, c, d, k, j, i)) mu = 0.0f;
-    a.lam[c][idx] = coef_at(p.em.decay[c], p.em.decay_full[c], idx) * mu;
-    const float src = coef_at(p.em.source[c], p.em.source_full[c], idx);
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int t = 2 * c + s;
-      if (a.scratch_e[t] == nullptr) continue;
-      float ld = (s == 0 ? src : -src) * mu;
-      if (p.cpml) ld = cpml_transpose(p.et[t], adj_axis(t), k, j, i, ld);
-      a.scratch_e[t][idx] = ld;
-    }
-    if (a.grad[c] != nullptr && k >= a.box_lo[0] && k < a.box_hi[0] && j >= a.box_lo[1] && j < a.box_hi[1] &&
-        i >= a.box_lo[2] && i < a.box_hi[2]) {
-      const int64_t b = (static_cast<int64_t>(k - a.box_lo[0]) * (a.box_hi[1] - a.box_lo[1]) + (j - a.box_lo[1])) *
-                            (a.box_hi[2] - a.box_lo[2]) +
-                        (i - a.box_lo[2]);
-      a.grad[c][b] += mu * a.curl[c][b];
-    }
-  }
+  const int idx = at(d, k, j, i);
+  float mu = a.lam[c][idx];
+  if (p.metallic && e_constrained(p.metallic, c, d, k, j, i)) mu = 0.0f;
+  const float src = coef_at(p.em.source[c], p.em.source_full[c], idx);
+  const float ld = (t % 2 == 0 ? src : -src) * mu;
+  return p.cpml ? cpml_transpose<false>(p.et[t], adj_axis(t), k, j, i, ld) : ld;
 }
 
-// 4b. B^T gather, per H site of component h.
-template <int h>
-__global__ void __launch_bounds__(kAdjThreads) adj_hgather_kernel(Step3D p, AdjDev a) {
-  const Dims d = component_dims(h, p.Z, p.Y, p.X);
-  const int64_t n = static_cast<int64_t>(d.z) * d.y * d.x;
+// lam_d of H term t at its H site, from the masked H adjoint field (what the H
+// pass left there) and the memory before its update.
+__device__ __forceinline__ float h_term(const Step3D& p, const AdjDev& a, int t, int k, int j, int i) {
+  const int h = t / 2;
+  const Dims d = component_dims(3 + h, p.Z, p.Y, p.X);
+  const int idx = at(d, k, j, i);
+  const float src = coef_at(p.hm.source[h], p.hm.source_full[h], idx);
+  const float ld = (t % 2 == 0 ? -src : src) * a.lam[3 + h][idx];
+  return p.cpml ? cpml_transpose<false>(p.ht[t], adj_axis(t), k, j, i, ld) : ld;
+}
+
+// The lattice points of a launch: a block covers 64 x 4 points of one plane.
+constexpr int kAdjX = 64, kAdjY = 4;
+
+// 4b + mask of 3a, per H site: lambda_H += B^T lam_d, then the PEC mask.
+template <int Active>
+__global__ void __launch_bounds__(kAdjX* kAdjY) adj_h_pass(const __grid_constant__ Step3D p,
+                                                           const __grid_constant__ AdjDev a) {
+  const int i = blockIdx.x * kAdjX + threadIdx.x, j = blockIdx.y * kAdjY + threadIdx.y;
   const float inv_res = 1.0f / p.res;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < n;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int k, j, i;
-    unflat(idx, d, k, j, i);
-    float acc = 0.0f;
+  for (int k = blockIdx.z; k <= p.Z; k += gridDim.z) {
 #pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      if (adj_e_src(t) != h || a.scratch_e[t] == nullptr) continue;
-      const int e = t / 2, axis = adj_axis(t);
-      const Dims de = component_dims(e, p.Z, p.Y, p.X);
-      const int N = axis == 0 ? d.z : (axis == 1 ? d.y : d.x);  // H samples; E has N + 1
-      const int m = coord_of(axis, k, j, i);
-      const bool lw = wall(p.metallic, axis, false), hw = wall(p.metallic, axis, true);
-      auto row = [&](int r) { return (r >= 1 && r <= N - 1) || (r == 0 && lw) || (r == N && hw); };
-      const int k1 = axis == 0 ? k + 1 : k, j1 = axis == 1 ? j + 1 : j, i1 = axis == 2 ? i + 1 : i;
-      const float t0 = row(m) ? a.scratch_e[t][lin(de, k, j, i)] : 0.0f;
-      const float t1 = row(m + 1) ? a.scratch_e[t][lin(de, k1, j1, i1)] : 0.0f;
-      // Derivative metrics: the backward difference at E coordinate m was
-      // scaled by metric_e[m] (and the ghost rows by metric_e[0] / [N]).
-      const float* me = p.metric_e[axis];
-      if (me != nullptr)
-        acc += t0 * me[m] - t1 * me[m + 1];
-      else
-        acc += (t0 - t1) * inv_res;
-    }
-    a.lam[h][idx] += acc;
-  }
-}
-
-// 3a. H transpose, per H site of component h.
-template <int h>
-__global__ void __launch_bounds__(kAdjThreads) adj_h_kernel(Step3D p, AdjDev a) {
-  const Dims d = component_dims(h, p.Z, p.Y, p.X);
-  const int64_t n = static_cast<int64_t>(d.z) * d.y * d.x;
-  const int hc = h - 3;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < n;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int k, j, i;
-    unflat(idx, d, k, j, i);
-    float mu = a.lam[h][idx];
-    if (h_constrained(p.metallic, h, d, k, j, i)) mu = 0.0f;
-    a.lam[h][idx] = coef_at(p.hm.decay[hc], p.hm.decay_full[hc], idx) * mu;
-    const float src = coef_at(p.hm.source[hc], p.hm.source_full[hc], idx);
+    for (int h = 3; h < 6; ++h) {
+      if (!((Active >> h) & 1)) continue;
+      const Dims d = component_dims(h, p.Z, p.Y, p.X);
+      if (k >= d.z || j >= d.y || i >= d.x) continue;
+      const int idx = at(d, k, j, i);
+      float acc = 0.0f;
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const int t = 2 * hc + s;
-      if (a.scratch_h[t] == nullptr) continue;
-      float ld = (s == 0 ? -src : src) * mu;
-      if (p.cpml) ld = cpml_transpose(p.ht[t], adj_axis(t), k, j, i, ld);
-      a.scratch_h[t][idx] = ld;
+      for (int t = 0; t < 6; ++t) {
+        if (adj_e_src(t) != h || !((Active >> (t / 2)) & 1)) continue;
+        const int axis = adj_axis(t);
+        const int N = axis == 0 ? d.z : (axis == 1 ? d.y : d.x);  // H samples; E has N + 1
+        const int m = coord_of(axis, k, j, i);
+        const bool lw = wall(p.metallic, axis, false), hw = wall(p.metallic, axis, true);
+        auto row = [&](int r) { return (r >= 1 && r <= N - 1) || (r == 0 && lw) || (r == N && hw); };
+        const int k1 = axis == 0 ? k + 1 : k, j1 = axis == 1 ? j + 1 : j, i1 = axis == 2 ? i + 1 : i;
+        const float t0 = row(m) ? e_term(p, a, t, k, j, i) : 0.0f;
+        const float t1 = row(m + 1) ? e_term(p, a, t, k1, j1, i1) : 0.0f;
+        // Derivative metrics: the backward difference at E coordinate m was
+        // scaled by metric_e[m] (and the ghost rows by metric_e[0] / [N]).
+        const float* me = p.metric_e[axis];
+        if (me != nullptr)
+          acc += t0 * me[m] - t1 * me[m + 1];
+        else
+          acc += (t0 - t1) * inv_res;
+      }
+      float lam = a.lam[h][idx] + acc;
+      if (p.metallic && h_constrained(p.metallic, h, d, k, j, i)) lam = 0.0f;
+      a.lam[h][idx] = lam;
     }
   }
 }
 
-// 3b. D^T gather, per E site of component e.
-template <int e>
-__global__ void __launch_bounds__(kAdjThreads) adj_egather_kernel(Step3D p, AdjDev a) {
-  const Dims d = component_dims(e, p.Z, p.Y, p.X);
-  const int64_t n = static_cast<int64_t>(d.z) * d.y * d.x;
+// 4a + 3b, per E site: mask, memories and identity part of the E transpose, the
+// design-box gradient, then lambda_E += D^T lam_d.
+template <int Active>
+__global__ void __launch_bounds__(kAdjX* kAdjY) adj_e_pass(const __grid_constant__ Step3D p,
+                                                           const __grid_constant__ AdjDev a) {
+  const int i = blockIdx.x * kAdjX + threadIdx.x, j = blockIdx.y * kAdjY + threadIdx.y;
   const float inv_res = 1.0f / p.res;
-  for (int64_t idx = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; idx < n;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    int k, j, i;
-    unflat(idx, d, k, j, i);
-    float acc = 0.0f;
+  for (int k = blockIdx.z; k <= p.Z; k += gridDim.z) {
 #pragma unroll
-    for (int t = 0; t < 6; ++t) {
-      if (adj_h_src(t) != e || a.scratch_h[t] == nullptr) continue;
-      const int hcomp = 3 + t / 2, axis = adj_axis(t);
-      const Dims dh = component_dims(hcomp, p.Z, p.Y, p.X);
-      const int N = axis == 0 ? dh.z : (axis == 1 ? dh.y : dh.x);
-      const int m = coord_of(axis, k, j, i);
-      const int k0 = axis == 0 ? k - 1 : k, j0 = axis == 1 ? j - 1 : j, i0 = axis == 2 ? i - 1 : i;
-      const float u_prev = m >= 1 ? a.scratch_h[t][lin(dh, k0, j0, i0)] : 0.0f;
-      const float u_here = m <= N - 1 ? a.scratch_h[t][lin(dh, k, j, i)] : 0.0f;
-      // Derivative metrics: the forward difference at H coordinate m was
-      // scaled by metric_h[m].
-      const float* mh = p.metric_h[axis];
-      if (mh != nullptr)
-        acc += (m >= 1 ? u_prev * mh[m - 1] : 0.0f) - (m <= N - 1 ? u_here * mh[m] : 0.0f);
-      else
-        acc += (u_prev - u_here) * inv_res;
+    for (int c = 0; c < 3; ++c) {
+      if (!((Active >> c) & 1)) continue;
+      const Dims d = component_dims(c, p.Z, p.Y, p.X);
+      if (k >= d.z || j >= d.y || i >= d.x) continue;
+      const int idx = at(d, k, j, i);
+      float mu = a.lam[c][idx];
+      if (p.metallic && e_constrained(p.metallic, c, d, k, j, i)) mu = 0.0f;
+      const float lam = coef_at(p.em.decay[c], p.em.decay_full[c], idx) * mu;
+      if (p.cpml) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          const int t = 2 * c + s;
+          if (!((Active >> adj_e_src(t)) & 1) || cpml_slot(p.et[t], coord_of(adj_axis(t), k, j, i)) < 0) continue;
+          const float src = coef_at(p.em.source[c], p.em.source_full[c], idx);
+          cpml_transpose<true>(p.et[t], adj_axis(t), k, j, i, (s == 0 ? src : -src) * mu);
+        }
+      }
+      if (a.grad[c] != nullptr && k >= a.box_lo[0] && k < a.box_hi[0] && j >= a.box_lo[1] && j < a.box_hi[1] &&
+          i >= a.box_lo[2] && i < a.box_hi[2]) {
+        const int64_t b = (static_cast<int64_t>(k - a.box_lo[0]) * (a.box_hi[1] - a.box_lo[1]) + (j - a.box_lo[1])) *
+                              (a.box_hi[2] - a.box_lo[2]) +
+                          (i - a.box_lo[2]);
+        a.grad[c][b] += mu * a.curl[c][b];
+      }
+      float acc = 0.0f;
+#pragma unroll
+      for (int t = 0; t < 6; ++t) {
+        if (adj_h_src(t) != c || !((Active >> (3 + t / 2)) & 1)) continue;
+        const int axis = adj_axis(t);
+        const Dims dh = component_dims(3 + t / 2, p.Z, p.Y, p.X);
+        const int N = axis == 0 ? dh.z : (axis == 1 ? dh.y : dh.x);
+        const int m = coord_of(axis, k, j, i);
+        const int k0 = axis == 0 ? k - 1 : k, j0 = axis == 1 ? j - 1 : j, i0 = axis == 2 ? i - 1 : i;
+        const float u_prev = m >= 1 ? h_term(p, a, t, k0, j0, i0) : 0.0f;
+        const float u_here = m <= N - 1 ? h_term(p, a, t, k, j, i) : 0.0f;
+        // Derivative metrics: the forward difference at H coordinate m was
+        // scaled by metric_h[m].
+        const float* mh = p.metric_h[axis];
+        if (mh != nullptr)
+          acc += (m >= 1 ? u_prev * mh[m - 1] : 0.0f) - (m <= N - 1 ? u_here * mh[m] : 0.0f);
+        else
+          acc += (u_prev - u_here) * inv_res;
+      }
+      a.lam[c][idx] = lam + acc;
     }
-    a.lam[e][idx] += acc;
+  }
+}
+
+// The rest of 3a, per H component (blockIdx.y): the memories, over the slabs;
+// and, where the H decay is not exactly 1, over every site with its scaling.
+template <int Active>
+__global__ void __launch_bounds__(kAdjThreads) adj_h_finish(const __grid_constant__ Step3D p,
+                                                            const __grid_constant__ AdjDev a) {
+  const int first = blockIdx.x * kAdjThreads + threadIdx.x, stride = gridDim.x * kAdjThreads;
+#pragma unroll
+  for (int hc = 0; hc < 3; ++hc) {
+    if (!((Active >> (3 + hc)) & 1) || static_cast<int>(blockIdx.y) != hc) continue;
+    const Dims d = component_dims(3 + hc, p.Z, p.Y, p.X);
+    auto advance = [&](int t, int k, int j, int i, float mu) {
+      const float src = coef_at(p.hm.source[hc], p.hm.source_full[hc], at(d, k, j, i));
+      cpml_transpose<true>(p.ht[t], adj_axis(t), k, j, i, (t % 2 == 0 ? -src : src) * mu);
+    };
+    const bool scaled = p.hm.decay_full[hc] || p.hm.decay[hc][0] != 1.0f;
+    if (!scaled) {
+      if (!p.cpml) continue;
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int t = 2 * hc + s, axis = adj_axis(t);
+        if (!((Active >> adj_h_src(t)) & 1)) continue;
+        const CpmlTermDev& term = p.ht[t];
+        const int w = term.low + term.high;
+        if (w == 0) continue;
+        const Dims sd = {axis == 0 ? w : d.z, axis == 1 ? w : d.y, axis == 2 ? w : d.x};  // the slab
+        const int n = sd.z * sd.y * sd.x;
+        for (int e = first; e < n; e += stride) {
+          const int r = e / sd.x;
+          int i = e - r * sd.x, k = r / sd.y, j = r - k * sd.y;
+          int& x = axis == 0 ? k : (axis == 1 ? j : i);
+          if (x >= term.low) x += term.n_axis - w;  // high slots
+          advance(t, k, j, i, a.lam[3 + hc][at(d, k, j, i)]);
+        }
+      }
+      continue;
+    }
+    const int n = d.z * d.y * d.x;
+    for (int e = first; e < n; e += stride) {
+      const int r = e / d.x;
+      const int i = e - r * d.x, k = r / d.y, j = r - k * d.y;
+      const float mu = a.lam[3 + hc][e];
+      if (p.cpml) {
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+          if ((Active >> adj_h_src(2 * hc + s)) & 1) advance(2 * hc + s, k, j, i, mu);
+      }
+      a.lam[3 + hc][e] = coef_at(p.hm.decay[hc], p.hm.decay_full[hc], e) * mu;
+    }
   }
 }
 
@@ -322,81 +369,41 @@ unsigned blocks_for(int64_t n) {
 
 }  // namespace
 
-cudaError_t launch_adjoint_step(cudaStream_t s, const Step3D& p, const DftDev* dft, const AdjDev& a, int active,
-                                int step) {
-  if (dft != nullptr && dft->monitor_count > 0 && dft->max_points > 0 && a.dft_grad_re != nullptr) {
-    if (dft->max_freqs > kAdjMaxFreqs) return cudaErrorInvalidValue;
-    const dim3 grid((dft->max_points + kAdjThreads - 1) / kAdjThreads, dft->monitor_count * 6, 1);
-    adj_dft_kernel<<<grid, kAdjThreads, 0, s>>>(*dft, a, step);
-  }
-  // One launch per active component and pass, in the component order of the
-  // transpose (E sites, B^T gathers, H sites, D^T gathers).
-  auto grid = [&](int c) {
-    const Dims d = component_dims(c, p.Z, p.Y, p.X);
-    return blocks_for(static_cast<int64_t>(d.z) * d.y * d.x);
-  };
-  if (active & 1) adj_e_kernel<0><<<grid(0), kAdjThreads, 0, s>>>(p, a);
-  if (active & 2) adj_e_kernel<1><<<grid(1), kAdjThreads, 0, s>>>(p, a);
-  if (active & 4) adj_e_kernel<2><<<grid(2), kAdjThreads, 0, s>>>(p, a);
-  if (active & 8) adj_hgather_kernel<3><<<grid(3), kAdjThreads, 0, s>>>(p, a);
-  if (active & 16) adj_hgather_kernel<4><<<grid(4), kAdjThreads, 0, s>>>(p, a);
-  if (active & 32) adj_hgather_kernel<5><<<grid(5), kAdjThreads, 0, s>>>(p, a);
-  if (active & 8) adj_h_kernel<3><<<grid(3), kAdjThreads, 0, s>>>(p, a);
-  if (active & 16) adj_h_kernel<4><<<grid(4), kAdjThreads, 0, s>>>(p, a);
-  if (active & 32) adj_h_kernel<5><<<grid(5), kAdjThreads, 0, s>>>(p, a);
-  if (active & 1) adj_egather_kernel<0><<<grid(0), kAdjThreads, 0, s>>>(p, a);
-  if (active & 2) adj_egather_kernel<1><<<grid(1), kAdjThreads, 0, s>>>(p, a);
-  if (active & 4) adj_egather_kernel<2><<<grid(2), kAdjThreads, 0, s>>>(p, a);
-  return cudaPeekAtLastError();
-}
-
-// ---- adjoint step without caller scratch -----------------------------------
-// The per-term scratch of fdtd_adjoint_step_noalloc lives in this one
-// file-scope device array (FDTD_ADJOINT_NOALLOC_MAX_FLOATS floats, 16 MiB),
-// so that entry point allocates no device memory.  Every call shares it:
-// calls that overlap on the GPU race.  Nothing in it needs clearing: each
-// call writes every scratch element it reads before reading it.
-static __device__ __align__(256) float g_adjoint_scratch[FDTD_ADJOINT_NOALLOC_MAX_FLOATS];
-
 namespace {
 
-// Device address of g_adjoint_scratch on the current device.  Looked up on
-// every call (a cheap runtime query) rather than cached, so that the address
-// stays right after the device's context is torn down and re-created (the
-// module, and with it the array, may then sit elsewhere).
-cudaError_t adjoint_scratch_address(float** out) {
-  void* p = nullptr;
-  const cudaError_t err = cudaGetSymbolAddress(&p, g_adjoint_scratch);
-  if (err != cudaSuccess) return err;
-  *out = static_cast<float*>(p);
-  return cudaSuccess;
+template <int Active>
+void launch_passes(cudaStream_t s, const Step3D& p, const AdjDev& a) {
+  const dim3 grid((p.X + kAdjX) / kAdjX, (p.Y + kAdjY) / kAdjY, p.Z + 1 < 65535 ? p.Z + 1 : 65535);
+  const dim3 block(kAdjX, kAdjY, 1);
+  adj_h_pass<Active><<<grid, block, 0, s>>>(p, a);
+  adj_e_pass<Active><<<grid, block, 0, s>>>(p, a);
+  // The slabs hold a few per cent of the sites.
+  const int64_t sites = static_cast<int64_t>(p.Z + 1) * (p.Y + 1) * (p.X + 1);
+  adj_h_finish<Active><<<dim3(blocks_for(sites / 4), 3, 1), kAdjThreads, 0, s>>>(p, a);
 }
 
 }  // namespace
 
-int64_t adjoint_noalloc_span(int64_t floats) { return (floats + 63) / 64 * 64; }
-
-cudaError_t launch_adjoint_step_noalloc(cudaStream_t s, const Step3D& p, const DftDev* dft, AdjDev a, int active,
-                                        int step, const int64_t e_len[6], const int64_t h_len[6]) {
-  int64_t need = 0;
-  for (int t = 0; t < 6; ++t) {
-    need += e_len[t] > 0 ? adjoint_noalloc_span(e_len[t]) : 0;
-    need += h_len[t] > 0 ? adjoint_noalloc_span(h_len[t]) : 0;
+cudaError_t launch_adjoint_steps(cudaStream_t s, const Step3D& p, const DftDev* dft, AdjDev a, int active, int step,
+                                 int count, int64_t curl_stride) {
+  const bool source = dft != nullptr && dft->monitor_count > 0 && dft->max_points > 0 && a.dft_grad_re != nullptr;
+  if (source && dft->max_freqs > kAdjMaxFreqs) return cudaErrorInvalidValue;
+  for (int n = 0; n < count; ++n) {
+    if (source) {
+      const dim3 grid((dft->max_points + kAdjThreads - 1) / kAdjThreads, dft->monitor_count * 6, 1);
+      adj_dft_kernel<<<grid, kAdjThreads, 0, s>>>(*dft, a, step - n);
+    }
+    switch (active) {
+      case kActive3D: launch_passes<kActive3D>(s, p, a); break;
+      case kActiveTM: launch_passes<kActiveTM>(s, p, a); break;
+      default: launch_passes<kActiveTE>(s, p, a); break;
+    }
+    const cudaError_t err = cudaPeekAtLastError();
+    if (err != cudaSuccess) return err;
+    for (int c = 0; c < 3; ++c)
+      if (a.curl[c] != nullptr) a.curl[c] -= curl_stride;
   }
-  if (need > FDTD_ADJOINT_NOALLOC_MAX_FLOATS) return cudaErrorInvalidValue;  // before any work
-  float* base = nullptr;
-  const cudaError_t err = adjoint_scratch_address(&base);
-  if (err != cudaSuccess) return err;
-  int64_t off = 0;
-  for (int t = 0; t < 6; ++t) {
-    a.scratch_e[t] = e_len[t] > 0 ? base + off : nullptr;
-    off += e_len[t] > 0 ? adjoint_noalloc_span(e_len[t]) : 0;
-  }
-  for (int t = 0; t < 6; ++t) {
-    a.scratch_h[t] = h_len[t] > 0 ? base + off : nullptr;
-    off += h_len[t] > 0 ? adjoint_noalloc_span(h_len[t]) : 0;
-  }
-  return launch_adjoint_step(s, p, dft, a, active, step);
+  return cudaSuccess;
 }
 
 cudaError_t launch_adjoint_curl(cudaStream_t s, const Step3D& p, const AdjDev& a, int active) {

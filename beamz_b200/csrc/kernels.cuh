@@ -148,20 +148,17 @@ cudaError_t launch_dft_flush(cudaStream_t s, const DftDev& dft, const float* sam
 // Adjoint step buffers (see FdtdAdjointStep in fdtd_b200.h).
 struct AdjDev {
   float* lam[6];           // adjoint fields, dense component shapes
-  float* scratch_e[6];     // per E term: lam_d at E sites
-  float* scratch_h[6];     // per H term: lam_d at H sites
   const float* dft_grad_re;
   const float* dft_grad_im;
   float* curl[3];          // forward curl over the design box
   float* grad[3];          // accumulated dJ/dc over the design box
   int box_lo[3], box_hi[3];
 };
-cudaError_t launch_adjoint_step(cudaStream_t s, const Step3D& p, const DftDev* dft, const AdjDev& a, int active,
-                                int step);
+// `count` adjoint steps from `step` downwards; a's curls are those of `step`,
+// each earlier step's `curl_stride` elements before.
+cudaError_t launch_adjoint_steps(cudaStream_t s, const Step3D& p, const DftDev* dft, AdjDev a, int active, int step,
+                                 int count, int64_t curl_stride);
 cudaError_t launch_adjoint_curl(cudaStream_t s, const Step3D& p, const AdjDev& a, int active);
-int64_t adjoint_noalloc_span(int64_t floats);
-cudaError_t launch_adjoint_step_noalloc(cudaStream_t s, const Step3D& p, const DftDev* dft, AdjDev a, int active,
-                                        int step, const int64_t e_len[6], const int64_t h_len[6]);
 
 // DFT arena view (see FdtdDft in fdtd_b200.h).
 struct DftDev {

@@ -938,7 +938,7 @@ bool f32_sized(const FdtdBuffer& b, int64_t n) { return is_f32(b) && b.data != n
 
 // Shared checks of an adjoint call: a valid dense phase program and a box
 // whose curl needs no ghost, wall or CPML handling.
-int check_adjoint(const FdtdProgram& p, const FdtdAdjointStep& a, const Layout& L, bool need_box) {
+int check_adjoint(const FdtdProgram& p, const FdtdAdjointStep& a, const Layout& L, bool need_box, int64_t steps = 1) {
   if (a.abi_version != FDTD_ABI_VERSION) return kInvalid;
   if (p.layout != FDTD_LAYOUT_DENSE) return kInvalid;
   const int64_t bz = a.box_hi[0] - a.box_lo[0], by = a.box_hi[1] - a.box_lo[1], bx = a.box_hi[2] - a.box_lo[2];
@@ -953,7 +953,7 @@ int check_adjoint(const FdtdProgram& p, const FdtdAdjointStep& a, const Layout& 
       if (a.curl[c].data != nullptr || a.grad[c].data != nullptr) return kInvalid;
       continue;
     }
-    if ((a.curl[c].data != nullptr && !f32_sized(a.curl[c], bz * by * bx)) ||
+    if ((a.curl[c].data != nullptr && !f32_sized(a.curl[c], steps * bz * by * bx)) ||
         (a.grad[c].data != nullptr && !f32_sized(a.grad[c], bz * by * bx)))
       return kInvalid;
     if (a.grad[c].data != nullptr && a.curl[c].data == nullptr) return kInvalid;
@@ -983,7 +983,8 @@ int check_adjoint(const FdtdProgram& p, const FdtdAdjointStep& a, const Layout& 
 
 // Elements of each derivative term's adjoint scratch (0 for a term between
 // inactive components): an E term's target E component, an H term's target H
-// component.  Both adjoint entry points size their scratch from this.
+// component.  The entry points check against this what a call declares; the
+// kernels need no scratch.
 void adjoint_term_lengths(const Layout& L, int64_t e_len[6], int64_t h_len[6]) {
   for (int t = 0; t < 6; ++t) {
     const int ec = kETermComp[t], hsrc = (t == 0 || t == 3) ? 5 : ((t == 1 || t == 4) ? 4 : 3);
@@ -1000,10 +1001,6 @@ void adjoint_term_lengths(const Layout& L, int64_t e_len[6], int64_t h_len[6]) {
 AdjDev adjoint_dev(const FdtdProgram& p, const FdtdAdjointStep& a) {
   AdjDev d{};
   for (int c = 0; c < 6; ++c) d.lam[c] = static_cast<float*>(p.fields[c].data);
-  for (int t = 0; t < 6; ++t) {
-    d.scratch_e[t] = static_cast<float*>(a.scratch_e[t].data);
-    d.scratch_h[t] = static_cast<float*>(a.scratch_h[t].data);
-  }
   d.dft_grad_re = static_cast<const float*>(a.dft_grad_re.data);
   d.dft_grad_im = static_cast<const float*>(a.dft_grad_im.data);
   for (int c = 0; c < 3; ++c) {
@@ -1018,65 +1015,64 @@ AdjDev adjoint_dev(const FdtdProgram& p, const FdtdAdjointStep& a) {
 }  // namespace
 }  // namespace fdtd
 
-int fdtd_adjoint_step(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a) {
-  if (adjoint == nullptr || a == nullptr) return fdtd::kInvalid;
+namespace fdtd {
+namespace {
+
+// What the three adjoint entry points share: validation (`steps` curls per
+// component), the DFT gradients, and the launches.  `scratch`: 0 = sized
+// scratch is declared, 1 = none and the declared bound holds, 2 = not looked at.
+int run_adjoint(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a, int scratch, int count) {
+  if (adjoint == nullptr || a == nullptr || count < 1) return kInvalid;
   FdtdProgram p = *adjoint;
   p.schedule = FDTD_SCHEDULE_PHASES;
-  if (p.material_kind != FDTD_MATERIAL_SITE) return fdtd::kInvalid;
-  const int v = fdtd::validate(p);
+  if (p.material_kind != FDTD_MATERIAL_SITE) return kInvalid;
+  const int v = validate(p);
   if (v != 0) return v;
-  fdtd::Layout L;
-  fdtd::layout_of(p, &L);
-  const int b = fdtd::check_adjoint(p, *a, L, false);
+  Layout L;
+  layout_of(p, &L);
+  const int b = check_adjoint(p, *a, L, false, count);
   if (b != 0) return b;
-  // Every derivative term between two active components needs its scratch.
-  int64_t e_len[6], h_len[6];
-  fdtd::adjoint_term_lengths(L, e_len, h_len);
+  int64_t e_len[6], h_len[6], need = 0;
+  adjoint_term_lengths(L, e_len, h_len);
   for (int t = 0; t < 6; ++t) {
-    if (e_len[t] > 0 ? !fdtd::f32_sized(a->scratch_e[t], e_len[t]) : a->scratch_e[t].data != nullptr)
-      return fdtd::kInvalid;
-    if (h_len[t] > 0 ? !fdtd::f32_sized(a->scratch_h[t], h_len[t]) : a->scratch_h[t].data != nullptr)
-      return fdtd::kInvalid;
+    if (scratch == 0) {
+      if (e_len[t] > 0 ? !f32_sized(a->scratch_e[t], e_len[t]) : a->scratch_e[t].data != nullptr) return kInvalid;
+      if (h_len[t] > 0 ? !f32_sized(a->scratch_h[t], h_len[t]) : a->scratch_h[t].data != nullptr) return kInvalid;
+    } else if (scratch == 1) {
+      if (a->scratch_e[t].data != nullptr || a->scratch_h[t].data != nullptr) return kInvalid;
+      need += (e_len[t] + 63) / 64 * 64 + (h_len[t] + 63) / 64 * 64;
+    }
   }
+  if (need > FDTD_ADJOINT_NOALLOC_MAX_FLOATS) return kInvalid;
   const bool dft = p.dft.monitor_count > 0 && a->dft_grad_re.data != nullptr;
-  fdtd::DftDev dd{};
+  DftDev dd{};
   if (dft) {
-    dd = fdtd::make_dft(p, p.fields);
-    if (!fdtd::f32_sized(a->dft_grad_re, dd.arena_len) || !fdtd::f32_sized(a->dft_grad_im, dd.arena_len))
-      return fdtd::kInvalid;
+    dd = make_dft(p, p.fields);
+    if (!f32_sized(a->dft_grad_re, dd.arena_len) || !f32_sized(a->dft_grad_im, dd.arena_len)) return kInvalid;
   }
-  const fdtd::Step3D sp = fdtd::make_step(p, L, 0, false, 0);
-  return static_cast<int>(fdtd::launch_adjoint_step(static_cast<cudaStream_t>(stream), sp, dft ? &dd : nullptr,
-                                                    fdtd::adjoint_dev(p, *a), L.active, a->step));
+  AdjDev d = adjoint_dev(p, *a);
+  const int64_t box = static_cast<int64_t>(a->box_hi[0] - a->box_lo[0]) * (a->box_hi[1] - a->box_lo[1]) *
+                      (a->box_hi[2] - a->box_lo[2]);
+  for (int c = 0; c < 3; ++c)
+    if (d.curl[c] != nullptr) d.curl[c] += (count - 1) * box;  // ascending steps: the last slice is a->step's
+  const Step3D sp = make_step(p, L, 0, false, 0);
+  return static_cast<int>(launch_adjoint_steps(static_cast<cudaStream_t>(stream), sp, dft ? &dd : nullptr, d, L.active,
+                                               a->step, count, box));
+}
+
+}  // namespace
+}  // namespace fdtd
+
+int fdtd_adjoint_step(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a) {
+  return fdtd::run_adjoint(stream, adjoint, a, 0, 1);
 }
 
 int fdtd_adjoint_step_noalloc(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a) {
-  if (adjoint == nullptr || a == nullptr) return fdtd::kInvalid;
-  FdtdProgram p = *adjoint;
-  p.schedule = FDTD_SCHEDULE_PHASES;
-  if (p.material_kind != FDTD_MATERIAL_SITE) return fdtd::kInvalid;
-  const int v = fdtd::validate(p);
-  if (v != 0) return v;
-  fdtd::Layout L;
-  fdtd::layout_of(p, &L);
-  const int b = fdtd::check_adjoint(p, *a, L, false);
-  if (b != 0) return b;
-  int64_t e_len[6], h_len[6];
-  fdtd::adjoint_term_lengths(L, e_len, h_len);
-  for (int t = 0; t < 6; ++t)
-    if (a->scratch_e[t].data != nullptr || a->scratch_h[t].data != nullptr) return fdtd::kInvalid;
-  // The scratch bound is checked once, by the launcher, before any work is enqueued.
-  const bool dft = p.dft.monitor_count > 0 && a->dft_grad_re.data != nullptr;
-  fdtd::DftDev dd{};
-  if (dft) {
-    dd = fdtd::make_dft(p, p.fields);
-    if (!fdtd::f32_sized(a->dft_grad_re, dd.arena_len) || !fdtd::f32_sized(a->dft_grad_im, dd.arena_len))
-      return fdtd::kInvalid;
-  }
-  const fdtd::Step3D sp = fdtd::make_step(p, L, 0, false, 0);
-  return static_cast<int>(fdtd::launch_adjoint_step_noalloc(static_cast<cudaStream_t>(stream), sp,
-                                                            dft ? &dd : nullptr, fdtd::adjoint_dev(p, *a), L.active,
-                                                            a->step, e_len, h_len));
+  return fdtd::run_adjoint(stream, adjoint, a, 1, 1);
+}
+
+int fdtd_adjoint_steps(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a, int32_t count) {
+  return fdtd::run_adjoint(stream, adjoint, a, 2, count);
 }
 
 int fdtd_adjoint_curl(void* stream, const FdtdProgram* forward, const FdtdAdjointStep* a) {

@@ -383,8 +383,8 @@ int fdtd_graph_destroy(void* graph);
 typedef struct FdtdAdjointStep {
   int32_t abi_version;
   int32_t step;              /* absolute step n whose transpose is applied */
-  FdtdBuffer scratch_e[6];   /* F32, per E term: that E component's shape */
-  FdtdBuffer scratch_h[6];   /* F32, per H term: that H component's shape */
+  FdtdBuffer scratch_e[6];   /* F32, per E term: that E component's shape (fdtd_adjoint_step; */
+  FdtdBuffer scratch_h[6];   /* per H term likewise): checked, no longer written */
   FdtdBuffer dft_grad_re;    /* F32 [arena], optional: dJ/d(dft re) */
   FdtdBuffer dft_grad_im;    /* F32 [arena], optional: dJ/d(dft im) */
   FdtdBuffer curl[3];        /* F32 [box], optional: forward curl of Ex/Ey/Ez over the box */
@@ -399,25 +399,26 @@ typedef struct FdtdAdjointStep {
  * the box (when grad/curl are given), then the H update's transpose. */
 int fdtd_adjoint_step(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a);
 
-/* Floats in the device scratch array of fdtd_adjoint_step_noalloc (16 MiB). */
+/* Largest program of fdtd_adjoint_step_noalloc, in scratch floats. */
 #define FDTD_ADJOINT_NOALLOC_MAX_FLOATS (4 * 1024 * 1024)
 
-/* fdtd_adjoint_step without caller scratch: the per-term scratch arrays are
- * carved from one device array of FDTD_ADJOINT_NOALLOC_MAX_FLOATS floats
- * inside this library, so the call allocates no device memory.  It is for
- * callers that cannot allocate device memory where they step the adjoint: a
- * host program that links only this C library and owns no device allocator
- * for temporaries, or one held to a fixed device-memory budget.
- * No counterpart in the reference (beamz differentiates through JAX).
- * a->scratch_e and a->scratch_h must be empty.  A program whose live
- * derivative terms need more scratch than the maximum (each term's array
- * rounded up to 64 floats; 2D TM up to about 1000 x 1000, 3D up to about
- * 330 000 lattice points) is rejected with cudaErrorInvalidValue (1) before
- * any work is enqueued.  Every call shares the one array: calls that overlap
- * on the GPU (two streams, or two host threads) race and corrupt each
- * other's results, so serialize them.  Nothing in it needs to start at
- * zero: each call writes every scratch element it reads first. */
+/* fdtd_adjoint_step without caller scratch, for callers that cannot allocate
+ * device memory where they step the adjoint: a host program that links only
+ * this C library and owns no device allocator for temporaries, or one held to
+ * a fixed device-memory budget.  No counterpart in the reference (beamz
+ * differentiates through JAX).  a->scratch_e and a->scratch_h must be empty.
+ * A program whose live derivative terms would fill more scratch than the
+ * maximum (each term's array rounded up to 64 floats; 2D TM up to about
+ * 1000 x 1000, 3D up to about 330 000 lattice points) is rejected with
+ * cudaErrorInvalidValue (1) before any work is enqueued; fdtd_adjoint_steps has
+ * no such bound. */
 int fdtd_adjoint_step_noalloc(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a);
+
+/* `count` adjoint steps in a row, a->step first, then each earlier one, enqueued
+ * by one call.  As fdtd_adjoint_step, without scratch, and with a->curl[c]
+ * holding the curls of steps a->step - count + 1 .. a->step in ascending order
+ * (F32 [count, box]). */
+int fdtd_adjoint_steps(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a, int32_t count);
 
 /* Write the forward curl of each active E component over `a`'s box into
  * a->curl from `forward`'s current H fields (call after a forward step). */
