@@ -914,7 +914,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           const float2 cy = Lossy ? sm.hcls[hc * 4 + 1] : make_float2(sm.hcoef[1], sm.hcoef[4]);
           const float2 cz = Lossy ? sm.hcls[hc * 4 + 2] : make_float2(sm.hcoef[2], sm.hcoef[5]);
           float hyv = h1<Exact>(HOy[b], cy.x, cy.y, d0, d1);
-          if (at_y0 && jc == 0 && wy0) hyv = 0.0f;
+          if ((at_y0 && jc == 0 && wy0) || (lyr && jc == Y && wy1)) hyv = 0.0f;
           float f0 = MH(E0y[b + 1] - E0y[b], 2, ih), f1 = MH(E0x[b + BX] - E0x[b], 1, jc);  // Hz: dEy/dx, dEx/dy
           if (AX && hz_ok) f0 = psi1_apply<Exact, 2>(p.ht[4], sm.cc[4], qc2, k, jc, ih, res, f0, false);
           if (AY && hz_ok) f1 = psi1_apply<Exact, 1>(p.ht[5], sm.cc[5], qc3, k, jc, ih, res, f1, false);
