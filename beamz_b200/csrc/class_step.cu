@@ -172,6 +172,11 @@ __device__ __forceinline__ float4 next4(float4 v, float n) { return make_float4(
 __device__ __forceinline__ float4 prev4(float p, float4 v) { return make_float4(p, v.x, v.y, v.z); }
 __device__ __forceinline__ float get(const float4& v, int q) { return q == 0 ? v.x : (q == 1 ? v.y : (q == 2 ? v.z : v.w)); }
 
+__device__ __forceinline__ void copy16(float* dst, const float* src) {
+  const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(at), "l"(src) : "memory");
+}
+
 // ---- arithmetic ------------------------------------------------------------
 // Exact: beamz's float32 order (kernels.py:458-626): every difference divided
 // by the cell size (correctly rounded, div_rn), every product and sum rounded
@@ -471,7 +476,13 @@ __device__ __forceinline__ float ghost_diff(float center, float below, int v, in
 // 8-warp CTAs: two per SM (shared memory), 128 registers; 4-warp CTAs: four.
 // Partial: X is not a multiple of 128 (the last tile is partial); only then
 // do the run-time bodies carry the per-lane store masks.
-template <int NW, bool Cpml, bool Exact, bool Lossy, bool Partial, bool Metric>
+// Site: one E coefficient per site and component (lossless materials with more
+// values than the codebook holds, and design runs that change them): three
+// float arrays on the field pitch take the place of the class ids.  A lane copies
+// its own cells' (16-byte cp.async) into its cells of the staged old H, which
+// nothing reads once its H is formed: in flight across the halo work and the
+// plane's barrier, at no registers and no shared memory.
+template <int NW, bool Cpml, bool Exact, bool Lossy, bool Partial, bool Metric, bool Site>
 __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
     class_step_kernel(const __grid_constant__ ClassMaps maps, const __grid_constant__ Step3D p) {
   using T = ClassTile<NW, Lossy>;
@@ -534,7 +545,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
   auto issue = [&](int q, int slot, bool first) {
     const int ne = (first ? 1 : 0) + (q + 1 <= Z ? 1 : 0);
     const unsigned bytes =
-        ne * 3 * T::EH * BX * 4 + 3 * T::HH * BX * 4 + T::IBOX + (xstage ? 4 * T::XW * T::HH * 4 : 0) +
+        ne * 3 * T::EH * BX * 4 + 3 * T::HH * BX * 4 + (Site ? 0 : T::IBOX) + (xstage ? 4 * T::XW * T::HH * 4 : 0) +
         (Lossy ? T::HIBYTES : 0);
     unsigned long long* b = &sm.bar[slot];
     tma::bar_expect(b, bytes);
@@ -544,7 +555,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
     if (q + 1 <= Z)
       for (int c = 0; c < 3; ++c) tma::load_3d(sm.e[(q + 1) % 3][c], &maps.e[c], i0 - 4, j0 - 1, q + 1, b);
     for (int c = 0; c < 3; ++c) tma::load_3d(sm.h[q % 2][c], &maps.h[c], i0 - 4, j0 - 1, q, b);
-    tma::load_3d(sm.ids[q % 2], &maps.ids, i0, j0, q, b);
+    if constexpr (!Site) tma::load_3d(sm.ids[q % 2], &maps.ids, i0, j0, q, b);
     if constexpr (Lossy) tma::load_3d(sm.hids[q % 2], &maps.hids, i0 - 16, j0 - 1, q, b);
     if (xstage) {
 #pragma unroll
@@ -560,7 +571,8 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     issue(kstart, 0, true);
   }
-  for (int e = tid; e < 256; e += T::NT) sm.cls[e] = p.class_coef[e];
+  if constexpr (!Site)
+    for (int e = tid; e < 256; e += T::NT) sm.cls[e] = p.class_coef[e];
   if constexpr (Lossy)
     for (int e = tid; e < 64 * 4; e += T::NT) sm.hcls[e] = p.h_class_coef[e];
   // CPML coefficient slabs, one (term, slot) per thread and round, so that every
@@ -854,6 +866,12 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           if (!zZ) st4m(p.hout[1] + o, hy, nvv);
           if (!rowY) st4m(p.hout[2] + o, hz, nvv);
         }
+        if constexpr (Site) {
+          if (emit && nvv > 0) {
+#pragma unroll
+            for (int n = 0; n < 3; ++n) copy16(&sm.h[hs][n][rc], p.site_c[n] + o);
+          }
+        }
         // ---- recomputed halo: row j0-1 (Hx by warp 0, Hz by warp 1) and
         //      column i0-1 (Hy, Hz by warp 2), read-only on psi ----
         if (halo_row_x && !zZ) {
@@ -996,13 +1014,22 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           fz0 = xtake(fz0, sm.xst[3][lane], sm.xd[1][warp]);
         }
         const float4 ex = ld4(E0x + rc), ey = ld4(E0y + rc), ez = ld4(E0z + rc);  // E(k) of the own cells
-        const uint32_t w4 = *reinterpret_cast<const uint32_t*>(IDS + warp * TX + 4 * lane);
+        const uint32_t w4 = Site ? 0u : *reinterpret_cast<const uint32_t*>(IDS + warp * TX + 4 * lane);
         float4 nx, ny, nz;
         if constexpr (Lossy) {
           const float2* ec = reinterpret_cast<const float2*>(sm.cls);
           nx = e4_loss<Exact>(ex, ec, w4, 0, fx0, fx1);
           ny = e4_loss<Exact>(ey, ec, w4, 1, fy0, fy1);
           nz = e4_loss<Exact>(ez, ec, w4, 2, fz0, fz1);
+        } else if constexpr (Site) {
+          asm volatile("cp.async.wait_all;\n" ::: "memory");  // this lane's own copies
+          const float4 sx = ld4(HOx + rc), sy = ld4(HOy + rc), sz = ld4(HOz + rc);
+          nx = make_float4(e_upd<Exact>(ex.x, sx.x, fx0.x, fx1.x), e_upd<Exact>(ex.y, sx.y, fx0.y, fx1.y),
+                           e_upd<Exact>(ex.z, sx.z, fx0.z, fx1.z), e_upd<Exact>(ex.w, sx.w, fx0.w, fx1.w));
+          ny = make_float4(e_upd<Exact>(ey.x, sy.x, fy0.x, fy1.x), e_upd<Exact>(ey.y, sy.y, fy0.y, fy1.y),
+                           e_upd<Exact>(ey.z, sy.z, fy0.z, fy1.z), e_upd<Exact>(ey.w, sy.w, fy0.w, fy1.w));
+          nz = make_float4(e_upd<Exact>(ez.x, sz.x, fz0.x, fz1.x), e_upd<Exact>(ez.y, sz.y, fz0.y, fz1.y),
+                           e_upd<Exact>(ez.z, sz.z, fz0.z, fz1.z), e_upd<Exact>(ez.w, sz.w, fz0.w, fz1.w));
         } else {
           const float4 t0 = sm.cls[w4 & 0xffu], t1 = sm.cls[(w4 >> 8) & 0xffu];
           const float4 t2 = sm.cls[(w4 >> 16) & 0xffu], t3 = sm.cls[w4 >> 24];
@@ -1118,8 +1145,9 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
         const float hz_y = sm.hn[2][rr - 1][cc], hx_y = sm.hn[0][rr - 1][cc];
         const float hz_x = sm.hn[2][rr][cc - 1], hy_x = sm.hn[1][rr][cc - 1];
         const bool in_box = cc >= 4 && cc < 4 + TX && rr >= 1 && rr <= TY;
-        const int cid = in_box ? IDS[(rr - 1) * TX + cc - 4] : p.site_class[(k * (Y + 1) + jj) * p.pitch8 + ii];
-        const float4 t = sm.cls[Lossy ? 0 : cid];
+        int cid = 0;
+        if constexpr (!Site) cid = in_box ? IDS[(rr - 1) * TX + cc - 4] : p.site_class[(k * (Y + 1) + jj) * p.pitch8 + ii];
+        const float4 t = Site ? make_float4(p.site_c[0][o], p.site_c[1][o], p.site_c[2][o], 0.0f) : sm.cls[Lossy ? 0 : cid];
         // E <- E + t.c (d0 - d1), or (Lossy) decay E + source (d0 - d1).
         auto eup = [&](float e, int n, float d0, float d1) {
           if constexpr (Lossy)
@@ -1220,7 +1248,7 @@ __device__ __forceinline__ float col_psi(const CpmlTermDev& t, int k, int j, int
   return slot >= 0 ? t.psi_in[psi_off<Axis>(t, slot, k, j, x)] : 0.0f;
 }
 
-template <bool Cpml, bool Exact, bool Lossy, bool Metric>
+template <bool Cpml, bool Exact, bool Lossy, bool Metric, bool Site>
 __global__ void __launch_bounds__(kColJ * kColK) class_column_kernel(const __grid_constant__ Step3D p) {
   __shared__ float hx[kColK + 1][kColJ + 1];  // new Hx at (k0 - 1 + a, j0 - 1 + b, X)
   __shared__ float amp[kMaxFusedSources];
@@ -1250,8 +1278,14 @@ __global__ void __launch_bounds__(kColJ * kColK) class_column_kernel(const __gri
   const bool ey_ok = live && j < Y, ez_ok = live && k < Z;
   const int o = live ? k * PL + j * P + X : 0;
   const float ey0 = ey_ok ? p.ein[1][o] : 0.0f, ez0 = ez_ok ? p.ein[2][o] : 0.0f;
-  const int cid = live ? p.site_class[(static_cast<int64_t>(k) * (Y + 1) + j) * p.pitch8 + X] : 0;
-  const float4 t = Lossy ? make_float4(0.f, 0.f, 0.f, 0.f) : p.class_coef[cid];
+  const int cid = !Site && live ? p.site_class[(static_cast<int64_t>(k) * (Y + 1) + j) * p.pitch8 + X] : 0;
+  float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+  if constexpr (Site) {
+    if (ey_ok) t.y = p.site_c[1][o];
+    if (ez_ok) t.z = p.site_c[2][o];
+  } else if constexpr (!Lossy) {
+    t = p.class_coef[cid];
+  }
   const float2* ec = reinterpret_cast<const float2*>(p.class_coef);  // Lossy: [128][4] (decay, source)
   // Lossy: the (decay, source) of H component n at lattice point (kk, jj, x).
   auto hco = [&](int kk, int jj, int x, int n) {
@@ -1355,20 +1389,21 @@ __global__ void __launch_bounds__(kColJ * kColK) class_column_kernel(const __gri
   }
 }
 
-template <int NW, bool Cpml, bool Exact, bool Lossy, bool Partial, bool Metric>
+template <int NW, bool Cpml, bool Exact, bool Lossy, bool Partial, bool Metric, bool Site>
 cudaError_t launch_class_p(cudaStream_t s, const ClassMaps& maps, const Step3D& p);
 
-template <int NW, bool Cpml, bool Exact, bool Lossy = false, bool Metric = false>
+template <int NW, bool Cpml, bool Exact, bool Lossy = false, bool Metric = false, bool Site = false>
 cudaError_t launch_class_t(cudaStream_t s, const ClassMaps& maps, const Step3D& p) {
-  if (p.X % ClassTile<NW, Lossy>::TX != 0) return launch_class_p<NW, Cpml, Exact, Lossy, true, Metric>(s, maps, p);
-  return launch_class_p<NW, Cpml, Exact, Lossy, false, Metric>(s, maps, p);
+  if (p.X % ClassTile<NW, Lossy>::TX != 0)
+    return launch_class_p<NW, Cpml, Exact, Lossy, true, Metric, Site>(s, maps, p);
+  return launch_class_p<NW, Cpml, Exact, Lossy, false, Metric, Site>(s, maps, p);
 }
 
-template <int NW, bool Cpml, bool Exact, bool Lossy, bool Partial, bool Metric>
+template <int NW, bool Cpml, bool Exact, bool Lossy, bool Partial, bool Metric, bool Site>
 cudaError_t launch_class_p(cudaStream_t s, const ClassMaps& maps, const Step3D& p) {
   using T = ClassTile<NW, Lossy>;
   const size_t smem = sizeof(typename T::Smem);
-  auto kern = class_step_kernel<NW, Cpml, Exact, Lossy, Partial, Metric>;
+  auto kern = class_step_kernel<NW, Cpml, Exact, Lossy, Partial, Metric, Site>;
   int device = 0;
   cudaError_t err = cudaGetDevice(&device);
   if (err != cudaSuccess) return err;
@@ -1405,7 +1440,7 @@ cudaError_t launch_class_p(cudaStream_t s, const ClassMaps& maps, const Step3D& 
   if (ctas > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
   {  // column X first: it reads only the step's inputs
     const dim3 cgrid((p.Y + 1 + kColJ - 1) / kColJ, (p.Z + 1 + kColK - 1) / kColK, 1);
-    class_column_kernel<Cpml, Exact, Lossy, Metric><<<cgrid, dim3(kColJ, kColK, 1), 0, s>>>(q);
+    class_column_kernel<Cpml, Exact, Lossy, Metric, Site><<<cgrid, dim3(kColJ, kColK, 1), 0, s>>>(q);
     err = cudaPeekAtLastError();
     if (err != cudaSuccess) return err;
   }
@@ -1427,7 +1462,7 @@ cudaError_t launch_class_shape(cudaStream_t s, const Step3D& p) {
       return cudaErrorInvalidValue;
   }
   const int64_t P8 = p.pitch8;
-  if (!tma::encode(&maps.ids, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.site_class, p.X + 1, p.Y + 1, p.Z + 1, P8,
+  if (!p.site && !tma::encode(&maps.ids, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.site_class, p.X + 1, p.Y + 1, p.Z + 1, P8,
                    P8 * (p.Y + 1), T::TX, T::TY))
     return cudaErrorInvalidValue;
   // Conductive material: the H classes, rows j0-1 .. and x from i0-16 (a
@@ -1455,6 +1490,9 @@ cudaError_t launch_class_shape(cudaStream_t s, const Step3D& p) {
     q.xstage = ok ? 1 : 0;
   }
   if constexpr (NW == 8) {
+    if (q.site)  // per-site coefficients: exact arithmetic, isotropic (validated)
+      return q.cpml ? launch_class_t<8, true, true, false, false, true>(s, maps, q)
+                    : launch_class_t<8, false, true, false, false, true>(s, maps, q);
     // Derivative metrics (axis-uniform / rectilinear grids): exact arithmetic
     // on lossless classes only (validated), 128 x 8 tiles.
     if (has_metric(q))
@@ -1470,9 +1508,9 @@ cudaError_t launch_class_shape(cudaStream_t s, const Step3D& p) {
 }  // namespace
 
 // tile_y: 8 (8 warps, 128 x 8 tiles) or 4 (4 warps, 128 x 4 tiles; programs
-// with derivative metrics always take 8).
+// with derivative metrics or per-site coefficients always take 8).
 cudaError_t launch_class_step(cudaStream_t s, const Step3D& p, int tile_y) {
-  return tile_y == 4 && !has_metric(p) ? launch_class_shape<4>(s, p) : launch_class_shape<8>(s, p);
+  return tile_y == 4 && !has_metric(p) && !p.site ? launch_class_shape<4>(s, p) : launch_class_shape<8>(s, p);
 }
 
 }  // namespace fdtd

@@ -66,6 +66,10 @@ struct Step3D {
   const uint8_t* site_class;
   int pitch8;
   const float4* class_coef;
+  // Per-site E coefficients (pitched FDTD_MATERIAL_SITE): Ex, Ey, Ez arrays on
+  // the field pitch, in place of the classes.
+  int site;
+  const float* site_c[3];
   int fast_math;  // tolerance arithmetic in the class step (1/dx folded, fused multiply-adds)
   // Class step dispatch order (longest first): tile rows [0, order[0]) and
   // [order[1], rows) and z chunks [0, order[2]) and [order[3], chunks) hold

@@ -104,8 +104,11 @@ int validate(const FdtdProgram& p) {
   const bool pitched = p.layout == FDTD_LAYOUT_PITCHED;
   if (p.layout != FDTD_LAYOUT_DENSE && !pitched) return kInvalid;
   if (pitched) {
-    // 3D codebook programs with uniform H coefficients; 16-byte-aligned rows.
-    if (p.ndim != 3 || p.material_kind != FDTD_MATERIAL_CODEBOOK) return kInvalid;
+    // 3D codebook programs, or lossless per-site ones, with uniform H
+    // coefficients; 16-byte-aligned rows.
+    if (p.ndim != 3 || p.material_kind == FDTD_MATERIAL_VOXEL) return kInvalid;
+    if (p.material_kind == FDTD_MATERIAL_SITE && (p.flags & (FDTD_FLAG_CLASSES | FDTD_FLAG_FAST_MATH | FDTD_FLAG_LOSSY)))
+      return kInvalid;
     if (p.pitch < L.X + 1 || p.pitch % 4 != 0) return kInvalid;
     if (static_cast<int64_t>(L.Z + 1) * (L.Y + 1) * p.pitch >= (int64_t{1} << 31)) return kInvalid;
   } else if (p.material_kind == FDTD_MATERIAL_CODEBOOK) {
@@ -124,7 +127,9 @@ int validate(const FdtdProgram& p) {
     if (p.schedule == FDTD_SCHEDULE_FUSED && !field_ok(p.fields_alt[c], n)) return kInvalid;
     if (pitched && (elements(p.h_decay[c % 3]) != 1 || elements(p.h_source_site[c % 3]) != 1)) return kInvalid;
     if (c < 3) {
-      if (p.material_kind == FDTD_MATERIAL_SITE &&
+      if (pitched && p.material_kind == FDTD_MATERIAL_SITE) {
+        if (!field_ok(p.e_source[c], n)) return kInvalid;  // a coefficient per site, on the fields' pitch
+      } else if (p.material_kind == FDTD_MATERIAL_SITE &&
           (!check_coeff(p.e_decay[c], n) || !check_coeff(p.e_source[c], n)))
         return kInvalid;
     } else {
@@ -400,7 +405,10 @@ Step3D make_step(const FdtdProgram& p, const Layout& L, int bank, bool fused, in
   s.cpml = p.cpml;
   for (int c = 0; c < 3; ++c) {
     const bool ea = (L.active >> c) & 1, ha = (L.active >> (c + 3)) & 1;
-    if (ea && p.material_kind == FDTD_MATERIAL_SITE) {
+    if (p.layout == FDTD_LAYOUT_PITCHED && p.material_kind == FDTD_MATERIAL_SITE) {
+      s.site = 1;
+      s.site_c[c] = static_cast<const float*>(p.e_source[c].data);
+    } else if (ea && p.material_kind == FDTD_MATERIAL_SITE) {
       s.em.decay[c] = static_cast<const float*>(p.e_decay[c].data);
       s.em.source[c] = static_cast<const float*>(p.e_source[c].data);
       s.em.decay_full[c] = elements(p.e_decay[c]) > 1;
@@ -699,7 +707,7 @@ cudaError_t enqueue_program(cudaStream_t s, const FdtdProgram& p) {
       for (int i = 0; i < n_hsrc; ++i) sp.hsrc[i] = hsrc[i];
       sp.n_esrc = n_esrc;
       for (int i = 0; i < n_esrc; ++i) sp.esrc[i] = esrc[i];
-      if (p.layout == FDTD_LAYOUT_PITCHED && (p.flags & FDTD_FLAG_CLASSES)) {
+      if (p.layout == FDTD_LAYOUT_PITCHED && (sp.site || (p.flags & FDTD_FLAG_CLASSES))) {
         err = launch_class_step(s, sp, p.tile_y);
       } else if (p.layout == FDTD_LAYOUT_PITCHED) {
         err = launch_fused_tma(s, sp, p.tile_y);

@@ -473,11 +473,25 @@ class DeviceProgram:
             raise ValueError("the pitched layout needs a 3D voxel or per-site program and the fused schedule; "
                              "conductive material or a non-isotropic grid also need the class step in exact "
                              "arithmetic")
+        # layout="site": the pitched layout with one E coefficient per site and
+        # component (lossless per-site material on an isotropic grid); "auto"
+        # takes it where the codebook does not hold the material's values.
+        site_ok = (site_sources is not None and schedule == "fused" and h_uniform and spec.metrics is None
+                   and arithmetic == "exact" and step_kernel == "classes")
+        if layout == "site" and not site_ok:
+            raise ValueError("the site layout needs a lossless per-site 3D program on an isotropic grid, the fused "
+                             "schedule and exact arithmetic")
+        self.per_site = layout == "site"
+        if self.per_site:
+            layout = "pitched"
+            nz, ny, nx = (int(v) for v in spec.grid_shape)
+            self.pitch = -(-(nx + 1) // 4) * 4
+            self.bank_shape = (nz + 1, ny + 1, self.pitch)
         f32 = np.float32
         dt_over_eps = f32(spec.dt) / f32(EPS_0)
         self.site_ids = self.site_coef = self.site_eps_table = None
         self._diag_eps = None
-        if layout in ("auto", "pitched") and pitched_ok:
+        if layout in ("auto", "pitched") and pitched_ok and not self.per_site:
             nz, ny, nx = (int(v) for v in spec.grid_shape)
             self.pitch = -(-(nx + 1) // 4) * 4
             self.bank_shape = (nz + 1, ny + 1, self.pitch)
@@ -494,7 +508,8 @@ class DeviceProgram:
             except CodebookOverflow:
                 if layout == "pitched":
                     raise
-                layout = "dense"
+                self.per_site = site_ok
+                layout = "pitched" if site_ok else "dense"
         elif layout == "auto" and not lossy_ok:
             layout = "dense"
         # Conductive (per-site decay) 3D programs: the class step with E and H
@@ -536,6 +551,8 @@ class DeviceProgram:
             raise ValueError("step_kernel is 'classes' or 'codebook'")
         if not self.lossy:
             self.site_class = self.class_coef = None
+        if self.per_site:
+            step_kernel = "site"
         if layout == "pitched" and step_kernel == "classes" and not self.lossy:
             try:
                 self.site_class, self.class_coef = device_site_classes(
@@ -551,7 +568,7 @@ class DeviceProgram:
                     step_kernel = "codebook"
         if layout != "pitched":
             step_kernel = "dense"
-        if step_kernel != "classes":
+        if step_kernel != "classes":  # the site step is exact too
             arithmetic = "exact"
         self.step_kernel = step_kernel
         self.arithmetic = arithmetic
@@ -603,7 +620,15 @@ class DeviceProgram:
             return abi.buffer_of(t)
 
         # Material.
-        if layout == "pitched":
+        if self.per_site:
+            s.material_kind = abi.FDTD_MATERIAL_SITE
+            for c in ("Ex", "Ey", "Ez"):
+                dz, dy, dx = self.shapes[c]
+                store = torch.zeros(self.bank_shape, dtype=torch.float32, device=dev)
+                self.e_source[c] = store[:dz, :dy, :dx]  # a view of the component's sites
+                self.e_source[c].copy_(_f32(site_sources[c], dev).expand(self.shapes[c]))
+                s.e_source[COMPONENT_INDEX[c]] = buf(store)
+        elif layout == "pitched":
             s.material_kind = abi.FDTD_MATERIAL_CODEBOOK
             s.site_ids = buf(self.site_ids)
             s.site_coef = buf(self.site_coef)
@@ -1027,7 +1052,7 @@ def field_diagnostics(state: DeviceState, program: DeviceProgram) -> FieldDiagno
                                torch.empty(18, dtype=torch.float64, device=dev))
     partials, out = state._diag_scratch
     d = abi.FdtdDiagnostics()
-    if program.layout == "pitched":
+    if program.layout == "pitched" and not program.per_site:
         if program.site_eps_table is None:
             raise ValueError("energy diagnostics of a conductive program need the spec's e_site_eps")
         d.site_eps_table = abi.buffer_of(program.site_eps_table)

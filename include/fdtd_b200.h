@@ -81,8 +81,12 @@ enum {
  * PITCHED: each component is a (Z+1, Y+1, pitch) float array, pitch a multiple
  *          of 4 and >= X+1, holding the component in its (dz, dy, dx) corner.
  *          All rows are 16-byte aligned, which lets the fused 3D step stage
- *          planes with TMA.  3D, FDTD_MATERIAL_CODEBOOK and uniform H
- *          coefficients only; fdtd_copy_component converts between layouts. */
+ *          planes with TMA.  3D and uniform H coefficients only, with
+ *          FDTD_MATERIAL_CODEBOOK, or with FDTD_MATERIAL_SITE for lossless
+ *          materials: e_source[c] then holds E <- E + source * curl's source on
+ *          the fields' (Z+1, Y+1, pitch) shape (e_decay is not read; isotropic
+ *          grids, exact arithmetic).  fdtd_copy_component converts between
+ *          layouts. */
 enum {
   FDTD_LAYOUT_DENSE = 0,
   FDTD_LAYOUT_PITCHED = 1,
