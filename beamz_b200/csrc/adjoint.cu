@@ -79,127 +79,265 @@ __device__ __forceinline__ float cpml_transpose(const CpmlTermDev& t, int axis, 
   return t.k[slot] * ld + t.a[slot] * acc;
 }
 
-// lam_d of E term t at its E site, from the E adjoint field before the E pass.
-__device__ __forceinline__ float e_term(const Step3D& p, const AdjDev& a, int t, int k, int j, int i) {
-  const int c = t / 2;
-  const Dims d = component_dims(c, p.Z, p.Y, p.X);
-  const int idx = at(d, k, j, i);
-  float mu = a.lam[c][idx];
-  if (p.metallic && e_constrained(p.metallic, c, d, k, j, i)) mu = 0.0f;
-  const float src = coef_at(p.em.source[c], p.em.source_full[c], idx);
-  const float ld = (t % 2 == 0 ? src : -src) * mu;
-  return p.cpml ? cpml_transpose<false>(p.et[t], adj_axis(t), k, j, i, ld) : ld;
+// Per axis: is this lattice point, with its neighbours one cell up and down, off
+// both faces and outside every slab?  Then the axis's terms need no ghost or
+// memory test.
+struct InnerAxes {
+  bool in[3];
+};
+__device__ __forceinline__ InnerAxes inner_axes(const Step3D& p, int k, int j, int i) {
+  auto in = [&](int axis, int c, int n) {
+    return c >= 1 && c <= n - 2 && c - 1 >= p.cpml_inner[axis][0] && c + 1 < p.cpml_inner[axis][1];
+  };
+  return {{in(0, k, p.Z), in(1, j, p.Y), in(2, i, p.X)}};
 }
 
-// lam_d of H term t at its H site, from the masked H adjoint field (what the H
-// pass left there) and the memory before its update.
-__device__ __forceinline__ float h_term(const Step3D& p, const AdjDev& a, int t, int k, int j, int i) {
-  const int h = t / 2;
-  const Dims d = component_dims(3 + h, p.Z, p.Y, p.X);
-  const int idx = at(d, k, j, i);
-  const float src = coef_at(p.hm.source[h], p.hm.source_full[h], idx);
-  const float ld = (t % 2 == 0 ? -src : src) * a.lam[3 + h][idx];
-  return p.cpml ? cpml_transpose<false>(p.ht[t], adj_axis(t), k, j, i, ld) : ld;
-}
-
-// The lattice points of a launch: a block covers 64 x 4 points of one plane.
+// The lattice points of a launch: a block covers 64 x 4 points of one plane, so
+// that z and y (and with them most slab tests) are uniform over a warp.  Written
+// term by term, with every site's offset, ghost, mask and slot test between its
+// loads, the passes issued 750-880 instructions per warp of points at 0.7 per
+// cycle (252 + 302 us at 256 x 256 x 128).  Here each site is read once, all
+// loads go out before the first test, and only the terms of an axis whose slab or
+// face is near are looked at further: 197 + 288 us.  What is left is the latency
+// of the slab points' chains, so the registers are held to eight blocks per SM
+// (at five: 192 + 345 us, at three: E pass 511 us).
 constexpr int kAdjX = 64, kAdjY = 4;
 
 // 4b + mask of 3a, per H site: lambda_H += B^T lam_d, then the PEC mask.
-template <int Active>
-__global__ void __launch_bounds__(kAdjX* kAdjY) adj_h_pass(const __grid_constant__ Step3D p,
-                                                           const __grid_constant__ AdjDev a) {
-  const int i = blockIdx.x * kAdjX + threadIdx.x, j = blockIdx.y * kAdjY + threadIdx.y;
-  const float inv_res = 1.0f / p.res;
-  for (int k = blockIdx.z; k <= p.Z; k += gridDim.z) {
-#pragma unroll
-    for (int h = 3; h < 6; ++h) {
-      if (!((Active >> h) & 1)) continue;
-      const Dims d = component_dims(h, p.Z, p.Y, p.X);
-      if (k >= d.z || j >= d.y || i >= d.x) continue;
-      const int idx = at(d, k, j, i);
+template <int Active, bool Metric>
+__device__ __forceinline__ void h_point(const Step3D& p, const AdjDev& a, float inv_res, int k, int j, int i) {
+  constexpr bool EX = Active & 1, EY = Active & 2, EZ = Active & 4, HX = Active & 8, HY = Active & 16, HZ = Active & 32;
+  const int Z = p.Z, Y = p.Y, X = p.X;
+  const bool kz = k < Z, jy = j < Y, ix = i < X;  // is there a neighbour one cell up?
+  const int nx = X + 1, ny = Y + 1;
+  const int ox = (k * ny + j) * X + i, oy = (k * Y + j) * nx + i, oz = (k * ny + j) * nx + i;
+  const int px = ny * X, py = Y * nx;  // planes of Ex (and Hy), Ey (and Hx)
+  // Every load first (at offset 0 where a site does not exist), with nothing that
+  // could branch between them; then masks and products.
+  struct Site {
+    float lam, src;
+  };
+  auto load = [&](int c, bool ok, int o) -> Site {
+    const int at = ok ? o : 0;
+    return {a.lam[c][at], coef_at(p.em.source[c], p.em.source_full[c], at)};
+  };
+  Site sx0{}, sxz{}, sxy{}, sy0{}, syz{}, syx{}, sz0{}, szy{}, szx{};
+  if constexpr (EX) {
+    sx0 = load(0, ix, ox);
+    if constexpr (HY) sxz = load(0, ix && kz, ox + px);
+    if constexpr (HZ) sxy = load(0, ix && jy, ox + X);
+  }
+  if constexpr (EY) {
+    sy0 = load(1, jy, oy);
+    if constexpr (HX) syz = load(1, jy && kz, oy + py);
+    if constexpr (HZ) syx = load(1, jy && ix, oy + 1);
+  }
+  if constexpr (EZ) {
+    sz0 = load(2, kz, oz);
+    if constexpr (HX) szy = load(2, kz && jy, oz + nx);
+    if constexpr (HY) szx = load(2, kz && ix, oz + 1);
+  }
+  const int oh = (k * Y + j) * X + i;                                 // Hz (Z + 1, Y, X)
+  const float lx = HX ? a.lam[3][kz && jy ? oy : 0] : 0.0f;           // Hx (Z, Y, X + 1): Ey's rows and planes
+  const float ly = HY ? a.lam[4][kz && ix ? ox : 0] : 0.0f;           // Hy (Z, Y + 1, X): Ex's
+  const float lz = HZ ? a.lam[5][jy && ix ? oh : 0] : 0.0f;
+  if (p.metallic) {
+    auto mask = [&](int c, Site& v, int kk, int jj, int ii) {
+      if (e_constrained(p.metallic, c, component_dims(c, Z, Y, X), kk, jj, ii)) v.lam = 0.0f;
+    };
+    mask(0, sx0, k, j, i), mask(0, sxz, k + 1, j, i), mask(0, sxy, k, j + 1, i);
+    mask(1, sy0, k, j, i), mask(1, syz, k + 1, j, i), mask(1, syx, k, j, i + 1);
+    mask(2, sz0, k, j, i), mask(2, szy, k, j + 1, i), mask(2, szx, k, j, i + 1);
+  }
+  // source * mask * lambda_E.
+  const float x0 = sx0.src * sx0.lam, xz = sxz.src * sxz.lam, xy = sxy.src * sxy.lam;
+  const float y0 = sy0.src * sy0.lam, yz = syz.src * syz.lam, yx = syx.src * syx.lam;
+  const float z0 = sz0.src * sz0.lam, zy = szy.src * szy.lam, zx = szx.src * szx.lam;
+  const InnerAxes in = inner_axes(p, k, j, i);
+  // lam_d of E term t at a site from its product, and 0 where the ghost makes B's
+  // row vanish.
+  auto ld = [&](int t, float v, int kk, int jj, int ii) -> float {
+    const int axis = adj_axis(t);
+    if (in.in[axis]) return v;
+    const int r = coord_of(axis, kk, jj, ii), N = axis == 0 ? Z : (axis == 1 ? Y : X);
+    if (!((r >= 1 && r <= N - 1) || (r == 0 && wall(p.metallic, axis, false)) || (r == N && wall(p.metallic, axis, true))))
+      return 0.0f;
+    return p.cpml ? cpml_transpose<false>(p.et[t], axis, kk, jj, ii, v) : v;
+  };
+  // Derivative metrics: the backward difference at E coordinate m was scaled by
+  // metric_e[m] (and the ghost rows by metric_e[0] / [N]).
+  auto gather = [&](int t, float t0, float t1) -> float {
+    if constexpr (Metric) {
+      const int axis = adj_axis(t), m = coord_of(axis, k, j, i);
+      return t0 * p.metric_e[axis][m] - t1 * p.metric_e[axis][m + 1];
+    } else {
+      return (t0 - t1) * inv_res;
+    }
+  };
+  if constexpr (HX) {
+    if (kz && jy) {
       float acc = 0.0f;
-#pragma unroll
-      for (int t = 0; t < 6; ++t) {
-        if (adj_e_src(t) != h || !((Active >> (t / 2)) & 1)) continue;
-        const int axis = adj_axis(t);
-        const int N = axis == 0 ? d.z : (axis == 1 ? d.y : d.x);  // H samples; E has N + 1
-        const int m = coord_of(axis, k, j, i);
-        const bool lw = wall(p.metallic, axis, false), hw = wall(p.metallic, axis, true);
-        auto row = [&](int r) { return (r >= 1 && r <= N - 1) || (r == 0 && lw) || (r == N && hw); };
-        const int k1 = axis == 0 ? k + 1 : k, j1 = axis == 1 ? j + 1 : j, i1 = axis == 2 ? i + 1 : i;
-        const float t0 = row(m) ? e_term(p, a, t, k, j, i) : 0.0f;
-        const float t1 = row(m + 1) ? e_term(p, a, t, k1, j1, i1) : 0.0f;
-        // Derivative metrics: the backward difference at E coordinate m was
-        // scaled by metric_e[m] (and the ghost rows by metric_e[0] / [N]).
-        const float* me = p.metric_e[axis];
-        if (me != nullptr)
-          acc += t0 * me[m] - t1 * me[m + 1];
-        else
-          acc += (t0 - t1) * inv_res;
-      }
-      float lam = a.lam[h][idx] + acc;
-      if (p.metallic && h_constrained(p.metallic, h, d, k, j, i)) lam = 0.0f;
-      a.lam[h][idx] = lam;
+      if constexpr (EY) acc += gather(2, ld(2, y0, k, j, i), ld(2, yz, k + 1, j, i));
+      if constexpr (EZ) acc += gather(5, ld(5, -z0, k, j, i), ld(5, -zy, k, j + 1, i));
+      float v = lx + acc;
+      if (p.metallic && h_constrained(p.metallic, 3, component_dims(3, Z, Y, X), k, j, i)) v = 0.0f;
+      a.lam[3][oy] = v;
+    }
+  }
+  if constexpr (HY) {
+    if (kz && ix) {
+      float acc = 0.0f;
+      if constexpr (EX) acc += gather(1, ld(1, -x0, k, j, i), ld(1, -xz, k + 1, j, i));
+      if constexpr (EZ) acc += gather(4, ld(4, z0, k, j, i), ld(4, zx, k, j, i + 1));
+      float v = ly + acc;
+      if (p.metallic && h_constrained(p.metallic, 4, component_dims(4, Z, Y, X), k, j, i)) v = 0.0f;
+      a.lam[4][ox] = v;
+    }
+  }
+  if constexpr (HZ) {
+    if (jy && ix) {
+      float acc = 0.0f;
+      if constexpr (EX) acc += gather(0, ld(0, x0, k, j, i), ld(0, xy, k, j + 1, i));
+      if constexpr (EY) acc += gather(3, ld(3, -y0, k, j, i), ld(3, -yx, k, j, i + 1));
+      float v = lz + acc;
+      if (p.metallic && h_constrained(p.metallic, 5, component_dims(5, Z, Y, X), k, j, i)) v = 0.0f;
+      a.lam[5][oh] = v;
     }
   }
 }
 
 // 4a + 3b, per E site: mask, memories and identity part of the E transpose, the
 // design-box gradient, then lambda_E += D^T lam_d.
-template <int Active>
-__global__ void __launch_bounds__(kAdjX* kAdjY) adj_e_pass(const __grid_constant__ Step3D p,
-                                                           const __grid_constant__ AdjDev a) {
-  const int i = blockIdx.x * kAdjX + threadIdx.x, j = blockIdx.y * kAdjY + threadIdx.y;
-  const float inv_res = 1.0f / p.res;
-  for (int k = blockIdx.z; k <= p.Z; k += gridDim.z) {
+template <int Active, bool Metric>
+__device__ __forceinline__ void e_point(const Step3D& p, const AdjDev& a, float inv_res, int k, int j, int i) {
+  constexpr bool EX = Active & 1, EY = Active & 2, EZ = Active & 4, HX = Active & 8, HY = Active & 16, HZ = Active & 32;
+  const int Z = p.Z, Y = p.Y, X = p.X;
+  const bool kz = k < Z, jy = j < Y, ix = i < X;     // is the point inside the H extent of an axis?
+  const bool kd = k >= 1, jd = j >= 1, id = i >= 1;  // is there a neighbour one cell down?
+  const int nx = X + 1, ny = Y + 1;
+  const int ox = (k * ny + j) * X + i, oy = (k * Y + j) * nx + i, oz = (k * ny + j) * nx + i, oh = (k * Y + j) * X + i;
+  const int px = ny * X, py = Y * nx;
+  // Every load first, as in h_point: source * lambda_H of the sites (masked by the
+  // H pass; 0 where there is none) and the own E values.
+  auto prod = [&](int h, bool ok, int o) -> float {
+    const int at = ok ? o : 0;
+    const float v = coef_at(p.hm.source[h], p.hm.source_full[h], at) * a.lam[3 + h][at];
+    return ok ? v : 0.0f;
+  };
+  const float ex = EX ? a.lam[0][ix ? ox : 0] : 0.0f, ey = EY ? a.lam[1][jy ? oy : 0] : 0.0f;
+  const float ez = EZ ? a.lam[2][kz ? oz : 0] : 0.0f;
+  const float dx = EX ? coef_at(p.em.decay[0], p.em.decay_full[0], ix ? ox : 0) : 0.0f;
+  const float dy = EY ? coef_at(p.em.decay[1], p.em.decay_full[1], jy ? oy : 0) : 0.0f;
+  const float dz = EZ ? coef_at(p.em.decay[2], p.em.decay_full[2], kz ? oz : 0) : 0.0f;
+  float x0 = 0.f, xz = 0.f, xy = 0.f, y0 = 0.f, yz = 0.f, yx = 0.f, z0 = 0.f, zy = 0.f, zx = 0.f;
+  if constexpr (HX) {
+    x0 = prod(0, kz && jy, oy);
+    if constexpr (EY) xz = prod(0, kd && jy, oy - py);
+    if constexpr (EZ) xy = prod(0, kz && jd, oy - nx);
+  }
+  if constexpr (HY) {
+    y0 = prod(1, kz && ix, ox);
+    if constexpr (EX) yz = prod(1, kd && ix, ox - px);
+    if constexpr (EZ) yx = prod(1, kz && id, ox - 1);
+  }
+  if constexpr (HZ) {
+    z0 = prod(2, jy && ix, oh);
+    if constexpr (EX) zy = prod(2, jd && ix, oh - X);
+    if constexpr (EY) zx = prod(2, jy && id, oh - 1);
+  }
+  const InnerAxes in = inner_axes(p, k, j, i);
+  const bool in_box = k >= a.box_lo[0] && k < a.box_hi[0] && j >= a.box_lo[1] && j < a.box_hi[1] && i >= a.box_lo[2] &&
+                      i < a.box_hi[2];
+  // lam_d of H term t at a site from its product (0 outside the H extent).
+  auto ld = [&](int t, float v, bool ok, int kk, int jj, int ii) -> float {
+    const int axis = adj_axis(t);
+    if (in.in[axis] || !p.cpml || !ok) return v;
+    return cpml_transpose<false>(p.ht[t], axis, kk, jj, ii, v);
+  };
+  // Derivative metrics: the forward difference at H coordinate m was scaled by
+  // metric_h[m].
+  auto gather = [&](int t, float prev, bool has_prev, float here, bool has_here) -> float {
+    if constexpr (Metric) {
+      const int axis = adj_axis(t), m = coord_of(axis, k, j, i);
+      return (has_prev ? prev * p.metric_h[axis][m - 1] : 0.0f) - (has_here ? here * p.metric_h[axis][m] : 0.0f);
+    } else {
+      return (prev - here) * inv_res;
+    }
+  };
+  // One E component: identity part, gather, memories, gradient.
+  auto site = [&](int c, int o, float mu, float dec, float acc) {
+    if (p.metallic && e_constrained(p.metallic, c, component_dims(c, Z, Y, X), k, j, i)) mu = 0.0f;
+    a.lam[c][o] = dec * mu + acc;
+    if (p.cpml) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      if (!((Active >> c) & 1)) continue;
-      const Dims d = component_dims(c, p.Z, p.Y, p.X);
-      if (k >= d.z || j >= d.y || i >= d.x) continue;
-      const int idx = at(d, k, j, i);
-      float mu = a.lam[c][idx];
-      if (p.metallic && e_constrained(p.metallic, c, d, k, j, i)) mu = 0.0f;
-      const float lam = coef_at(p.em.decay[c], p.em.decay_full[c], idx) * mu;
-      if (p.cpml) {
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const int t = 2 * c + s;
-          if (!((Active >> adj_e_src(t)) & 1) || cpml_slot(p.et[t], coord_of(adj_axis(t), k, j, i)) < 0) continue;
-          const float src = coef_at(p.em.source[c], p.em.source_full[c], idx);
-          cpml_transpose<true>(p.et[t], adj_axis(t), k, j, i, (s == 0 ? src : -src) * mu);
-        }
+      for (int s = 0; s < 2; ++s) {
+        const int t = 2 * c + s, axis = adj_axis(t);
+        if (in.in[axis] || !((Active >> adj_e_src(t)) & 1) || cpml_slot(p.et[t], coord_of(axis, k, j, i)) < 0) continue;
+        const float src = coef_at(p.em.source[c], p.em.source_full[c], o);
+        cpml_transpose<true>(p.et[t], axis, k, j, i, (s == 0 ? src : -src) * mu);
       }
-      if (a.grad[c] != nullptr && k >= a.box_lo[0] && k < a.box_hi[0] && j >= a.box_lo[1] && j < a.box_hi[1] &&
-          i >= a.box_lo[2] && i < a.box_hi[2]) {
-        const int64_t b = (static_cast<int64_t>(k - a.box_lo[0]) * (a.box_hi[1] - a.box_lo[1]) + (j - a.box_lo[1])) *
-                              (a.box_hi[2] - a.box_lo[2]) +
-                          (i - a.box_lo[2]);
-        a.grad[c][b] += mu * a.curl[c][b];
-      }
+    }
+    if (in_box && a.grad[c] != nullptr) {
+      const int64_t b = (static_cast<int64_t>(k - a.box_lo[0]) * (a.box_hi[1] - a.box_lo[1]) + (j - a.box_lo[1])) *
+                            (a.box_hi[2] - a.box_lo[2]) +
+                        (i - a.box_lo[2]);
+      a.grad[c][b] += mu * a.curl[c][b];
+    }
+  };
+  if constexpr (EX) {
+    if (ix) {
       float acc = 0.0f;
-#pragma unroll
-      for (int t = 0; t < 6; ++t) {
-        if (adj_h_src(t) != c || !((Active >> (3 + t / 2)) & 1)) continue;
-        const int axis = adj_axis(t);
-        const Dims dh = component_dims(3 + t / 2, p.Z, p.Y, p.X);
-        const int N = axis == 0 ? dh.z : (axis == 1 ? dh.y : dh.x);
-        const int m = coord_of(axis, k, j, i);
-        const int k0 = axis == 0 ? k - 1 : k, j0 = axis == 1 ? j - 1 : j, i0 = axis == 2 ? i - 1 : i;
-        const float u_prev = m >= 1 ? h_term(p, a, t, k0, j0, i0) : 0.0f;
-        const float u_here = m <= N - 1 ? h_term(p, a, t, k, j, i) : 0.0f;
-        // Derivative metrics: the forward difference at H coordinate m was
-        // scaled by metric_h[m].
-        const float* mh = p.metric_h[axis];
-        if (mh != nullptr)
-          acc += (m >= 1 ? u_prev * mh[m - 1] : 0.0f) - (m <= N - 1 ? u_here * mh[m] : 0.0f);
-        else
-          acc += (u_prev - u_here) * inv_res;
-      }
-      a.lam[c][idx] = lam + acc;
+      if constexpr (HY) acc += gather(2, ld(2, -yz, kd, k - 1, j, i), kd, ld(2, -y0, kz, k, j, i), kz);
+      if constexpr (HZ) acc += gather(5, ld(5, zy, jd, k, j - 1, i), jd, ld(5, z0, jy, k, j, i), jy);
+      site(0, ox, ex, dx, acc);
     }
   }
+  if constexpr (EY) {
+    if (jy) {
+      float acc = 0.0f;
+      if constexpr (HX) acc += gather(1, ld(1, xz, kd, k - 1, j, i), kd, ld(1, x0, kz, k, j, i), kz);
+      if constexpr (HZ) acc += gather(4, ld(4, -zx, id, k, j, i - 1), id, ld(4, -z0, ix, k, j, i), ix);
+      site(1, oy, ey, dy, acc);
+    }
+  }
+  if constexpr (EZ) {
+    if (kz) {
+      float acc = 0.0f;
+      if constexpr (HX) acc += gather(0, ld(0, -xy, jd, k, j - 1, i), jd, ld(0, -x0, jy, k, j, i), jy);
+      if constexpr (HY) acc += gather(3, ld(3, yx, id, k, j, i - 1), id, ld(3, y0, ix, k, j, i), ix);
+      site(2, oz, ez, dz, acc);
+    }
+  }
+}
+
+// Blocks stride over rows and planes beyond the launch limits; a 2D program lives
+// on plane 0.
+template <int Active, bool Metric>
+__global__ void __launch_bounds__(kAdjX* kAdjY, 8) adj_h_pass(const __grid_constant__ Step3D p,
+                                                              const __grid_constant__ AdjDev a) {
+  const int i = blockIdx.x * kAdjX + threadIdx.x;
+  if (i > p.X) return;
+  const float inv_res = 1.0f / p.res;
+  const int planes = Active == kActive3D ? p.Z + 1 : 1;
+#pragma unroll 1
+  for (int k = blockIdx.z; k < planes; k += gridDim.z)
+#pragma unroll 1
+    for (int j = blockIdx.y * kAdjY + threadIdx.y; j <= p.Y; j += gridDim.y * kAdjY)
+      h_point<Active, Metric>(p, a, inv_res, k, j, i);
+}
+
+template <int Active, bool Metric>
+__global__ void __launch_bounds__(kAdjX* kAdjY, 8) adj_e_pass(const __grid_constant__ Step3D p,
+                                                              const __grid_constant__ AdjDev a) {
+  const int i = blockIdx.x * kAdjX + threadIdx.x;
+  if (i > p.X) return;
+  const float inv_res = 1.0f / p.res;
+  const int planes = Active == kActive3D ? p.Z + 1 : 1;
+#pragma unroll 1
+  for (int k = blockIdx.z; k < planes; k += gridDim.z)
+#pragma unroll 1
+    for (int j = blockIdx.y * kAdjY + threadIdx.y; j <= p.Y; j += gridDim.y * kAdjY)
+      e_point<Active, Metric>(p, a, inv_res, k, j, i);
 }
 
 // The rest of 3a, per H component (blockIdx.y): the memories, over the slabs;
@@ -373,10 +511,16 @@ namespace {
 
 template <int Active>
 void launch_passes(cudaStream_t s, const Step3D& p, const AdjDev& a) {
-  const dim3 grid((p.X + kAdjX) / kAdjX, (p.Y + kAdjY) / kAdjY, p.Z + 1 < 65535 ? p.Z + 1 : 65535);
+  const auto capped = [](int n) { return static_cast<unsigned>(n < 65535 ? n : 65535); };
+  const dim3 grid((p.X + kAdjX) / kAdjX, capped((p.Y + kAdjY) / kAdjY), Active != kActive3D ? 1 : capped(p.Z + 1));
   const dim3 block(kAdjX, kAdjY, 1);
-  adj_h_pass<Active><<<grid, block, 0, s>>>(p, a);
-  adj_e_pass<Active><<<grid, block, 0, s>>>(p, a);
+  if (has_metric(p)) {
+    adj_h_pass<Active, true><<<grid, block, 0, s>>>(p, a);
+    adj_e_pass<Active, true><<<grid, block, 0, s>>>(p, a);
+  } else {
+    adj_h_pass<Active, false><<<grid, block, 0, s>>>(p, a);
+    adj_e_pass<Active, false><<<grid, block, 0, s>>>(p, a);
+  }
   // The slabs hold a few per cent of the sites.
   const int64_t sites = static_cast<int64_t>(p.Z + 1) * (p.Y + 1) * (p.X + 1);
   adj_h_finish<Active><<<dim3(blocks_for(sites / 4), 3, 1), kAdjThreads, 0, s>>>(p, a);
