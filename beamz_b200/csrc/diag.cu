@@ -10,6 +10,8 @@
 // and shared-memory block reductions, and a fixed partition and summation
 // order, so a result is identical from run to run.
 
+#include <cooperative_groups.h>
+
 #include "kernels.cuh"
 
 namespace fdtd {
@@ -51,13 +53,17 @@ __device__ __forceinline__ void block_reduce(double& s, float& m, unsigned& n) {
 
 // Rows (k, j) of one component, one warp per row: warp w of block b sweeps
 // rows b * warps_per_block + w, then + all warps of the grid; its lanes stride
-// along x, eight loads in flight each.  A lane forms each product eps * v^2 in
-// float and sums its products of a row in float; each row then enters the
-// double accumulator once, weighted by its y/z factor, with the two end sites
-// of an edge-aligned x axis taken at half weight.  MAT: 0 eps_r = 1, 1
-// codebook ids and table, 2 per-site array.
-template <int MAT>
-__device__ __forceinline__ void diag_rows(const DiagComp& q, double& s, float& mx, unsigned& bad) {
+// along x.  A lane forms each product eps * v^2 in float and sums its products
+// of a row in float; each row then enters the double accumulator once, weighted
+// by its y/z factor, with the two end sites of an edge-aligned x axis taken at
+// half weight.  MAT: 0 eps_r = 1, 1 codebook ids and table (in shared memory), 2
+// per-site array.  Vec: rows start on 16 bytes (the pitched layout), so a lane
+// takes four sites per load; the sweep is a plain read of the fields and ids,
+// and with 4-byte loads and a table gather per site it took 443 us at 384 x 384 x
+// 192 (1.0 GB with the ids read per component; 282 us now).
+template <int MAT, bool Vec>
+__device__ __forceinline__ void diag_rows(const DiagComp& q, const float* table, double& s, float& mx, unsigned& bad) {
+  constexpr int N = Vec ? 4 : 1;
   const int rows = q.d.z * q.d.y;  // < 2^31: component arrays are validated below 2^31 elements
   const int lane = threadIdx.x & 31;
   const int step = gridDim.x * kDiagWarps;
@@ -66,20 +72,36 @@ __device__ __forceinline__ void diag_rows(const DiagComp& q, double& s, float& m
     const int64_t base = k * q.plane + j * q.row;
     const float* f = q.field + base;
     float acc = 0.0f, ends = 0.0f;
-#pragma unroll 8
-    for (int i = lane; i < q.d.x; i += 32) {
-      const float x = f[i];
-      float e = 1.0f;
-      if constexpr (MAT == 1) e = q.table[(q.ids[base + i] >> q.shift) & 0xffu];
-      if constexpr (MAT == 2) e = q.eps[static_cast<int64_t>(r) * q.d.x + i];
-      if (!isfinite(x)) {
-        ++bad;
-        continue;
+#pragma unroll 4
+    for (int i0 = lane * N; i0 < q.d.x; i0 += 32 * N) {
+      float x[N];
+      uint32_t id[N];
+      if constexpr (Vec) {
+        const float4 v = *reinterpret_cast<const float4*>(f + i0);
+        x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+        if constexpr (MAT == 1) {
+          const uint4 w = *reinterpret_cast<const uint4*>(q.ids + base + i0);
+          id[0] = w.x, id[1] = w.y, id[2] = w.z, id[3] = w.w;
+        }
+      } else {
+        x[0] = f[i0];
+        if constexpr (MAT == 1) id[0] = q.ids[base + i0];
       }
-      mx = fmaxf(mx, fabsf(x));
-      const float prod = e * x * x;
-      acc += prod;
-      if (i == 0 || i == q.d.x - 1) ends += prod;
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        const int i = i0 + n;
+        const bool in = !Vec || i < q.d.x;  // the row's padding holds anything
+        float e = 1.0f;
+        if constexpr (MAT == 1) e = table[(id[n] >> q.shift) & 0xffu];
+        if constexpr (MAT == 2) e = in ? q.eps[static_cast<int64_t>(r) * q.d.x + i] : 0.0f;
+        const bool ok = isfinite(x[n]);
+        bad += in && !ok;
+        const float v = in && ok ? x[n] : 0.0f;
+        mx = fmaxf(mx, fabsf(v));
+        const float prod = in && ok ? e * v * v : 0.0f;
+        acc += prod;
+        if (i == 0 || i == q.d.x - 1) ends += prod;
+      }
     }
     double h = 1.0;
     if (q.integrate_z && q.edge_z && (k == 0 || k == q.d.z - 1)) h *= 0.5;
@@ -89,15 +111,22 @@ __device__ __forceinline__ void diag_rows(const DiagComp& q, double& s, float& m
 }
 
 __global__ void __launch_bounds__(kDiagThreads) diag_partial_kernel(DiagArgs a) {
+  __shared__ float table[256];
   const int c = blockIdx.y;
   double s = 0.0;
   float mx = 0.0f;
   unsigned bad = 0;
   if ((a.active >> c) & 1) {
     const DiagComp& q = a.comp[c];
-    if (q.ids) diag_rows<1>(q, s, mx, bad);
-    else if (q.eps) diag_rows<2>(q, s, mx, bad);
-    else diag_rows<0>(q, s, mx, bad);
+    if (q.ids) {
+      for (int e = threadIdx.x; e < 256; e += kDiagThreads) table[e] = q.table[e];
+      __syncthreads();
+    }
+    const bool vec = q.row % 4 == 0 && q.plane % 4 == 0 && q.row >= (q.d.x + 3) / 4 * 4 &&
+                     (reinterpret_cast<uintptr_t>(q.field) & 15) == 0 && (reinterpret_cast<uintptr_t>(q.ids) & 15) == 0;
+    if (q.ids) vec ? diag_rows<1, true>(q, table, s, mx, bad) : diag_rows<1, false>(q, table, s, mx, bad);
+    else if (q.eps) vec ? diag_rows<2, true>(q, table, s, mx, bad) : diag_rows<2, false>(q, table, s, mx, bad);
+    else vec ? diag_rows<0, true>(q, table, s, mx, bad) : diag_rows<0, false>(q, table, s, mx, bad);
   }
   block_reduce(s, mx, bad);
   if (threadIdx.x == 0) {
@@ -128,11 +157,18 @@ __global__ void __launch_bounds__(kDiagThreads) diag_final_kernel(const double* 
   }
 }
 
-// One block per (monitor, component, frequency): squared norms of the change,
-// the current and the previous vector, then prev <- current.
-__global__ void __launch_bounds__(kDiagThreads) dft_change_kernel(DftDev d, float* prev_re, float* prev_im,
-                                                                  double* out) {
-  const int key = blockIdx.x;
+// A cluster of eight blocks per (monitor, component, frequency): squared norms
+// of the change, the current and the previous vector, then prev <- current.  The
+// cluster's first block adds the blocks' sums in order.  (One block per vector
+// left most SMs idle: 90 vectors of 60 k points took 134 us, now 32 us.)
+constexpr int kChangeBlocks = 8;
+
+__global__ void __cluster_dims__(kChangeBlocks, 1, 1) __launch_bounds__(kDiagThreads)
+    dft_change_kernel(DftDev d, float* prev_re, float* prev_im, double* out) {
+  __shared__ double total[3];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int part = blockIdx.x % kChangeBlocks, key = blockIdx.x / kChangeBlocks;
   const int f = key % d.max_freqs, mc = key / d.max_freqs;
   const int m = mc / 6, c = mc % 6;
   const int* cnt = d.counts + 5 * m;
@@ -144,7 +180,7 @@ __global__ void __launch_bounds__(kDiagThreads) dft_change_kernel(DftDev d, floa
                   voff + static_cast<int64_t>(6) * nf * np <= d.arena_len;
   if (on) {
     const int64_t base = voff + (static_cast<int64_t>(c) * nf + f) * np;
-    for (int p = threadIdx.x; p < np; p += kDiagThreads) {
+    for (int p = part * kDiagThreads + threadIdx.x; p < np; p += kChangeBlocks * kDiagThreads) {
       const float re = d.re[base + p], im = d.im[base + p];
       const double dr = static_cast<double>(re) - prev_re[base + p], di = static_cast<double>(im) - prev_im[base + p];
       const double pr = prev_re[base + p], pi = prev_im[base + p];
@@ -165,10 +201,17 @@ __global__ void __launch_bounds__(kDiagThreads) dft_change_kernel(DftDev d, floa
   __syncthreads();
   block_reduce(pp, unused, none);
   if (threadIdx.x == 0) {
-    out[key * 3 + 0] = dd;
-    out[key * 3 + 1] = cc;
-    out[key * 3 + 2] = pp;
+    total[0] = dd;
+    total[1] = cc;
+    total[2] = pp;
   }
+  cluster.sync();
+  if (part == 0 && threadIdx.x < 3) {
+    double sum = 0.0;
+    for (int b = 0; b < kChangeBlocks; ++b) sum += *cluster.map_shared_rank(&total[threadIdx.x], b);
+    out[key * 3 + threadIdx.x] = sum;
+  }
+  cluster.sync();  // no block leaves while its sums are read
 }
 
 }  // namespace
@@ -184,7 +227,7 @@ cudaError_t launch_field_diagnostics(cudaStream_t s, const DiagArgs& a, double* 
 cudaError_t launch_dft_change(cudaStream_t s, const DftDev& d, float* prev_re, float* prev_im, double* out) {
   const int keys = d.monitor_count * 6 * d.max_freqs;
   if (keys <= 0) return cudaSuccess;
-  dft_change_kernel<<<keys, kDiagThreads, 0, s>>>(d, prev_re, prev_im, out);
+  dft_change_kernel<<<keys * kChangeBlocks, kDiagThreads, 0, s>>>(d, prev_re, prev_im, out);
   return cudaPeekAtLastError();
 }
 
