@@ -347,10 +347,9 @@ def eps_to_coefficients_2d(eps_voxels, dt, eps0):
     """TM Ez coefficient c = dt / (eps0 eps_site), the site taking its owning
     voxel (beamz/lattice.py:935-972), as differentiable torch ops."""
     torch = _torch()
-    ny, nx = eps_voxels.shape
-    rows = torch.clamp(torch.arange(ny + 1, device=eps_voxels.device), max=ny - 1)
-    cols = torch.clamp(torch.arange(nx + 1, device=eps_voxels.device), max=nx - 1)
-    site = eps_voxels[rows][:, cols]
+    # The last voxel row and column also own the sites beyond them.
+    site = torch.cat([eps_voxels, eps_voxels[-1:]], dim=0)
+    site = torch.cat([site, site[:, -1:]], dim=1)
     return torch.tensor(np.float32(dt), device=eps_voxels.device) / (
         torch.tensor(np.float32(eps0), device=eps_voxels.device) * site)
 
@@ -360,25 +359,17 @@ def eps_to_coefficients_3d(eps_voxels, dt, eps0):
     of the four voxels sharing each edge with clipped indices
     (beamz/lattice.py:732-786), c = fl(dt)/fl(eps0) * (1/eps_site)."""
     torch = _torch()
-    nz, ny, nx = eps_voxels.shape
     dev = eps_voxels.device
 
-    def clip_idx(n, m):
-        return torch.clamp(torch.arange(-1, n, device=dev), 0, m - 1), torch.clamp(torch.arange(0, n + 1, device=dev), 0, m - 1)
+    def pair(v, dim):  # the mean of each site's lower and upper voxel, clipped at the faces
+        lo = torch.cat([v.narrow(dim, 0, 1), v], dim=dim)
+        hi = torch.cat([v, v.narrow(dim, v.shape[dim] - 1, 1)], dim=dim)
+        return 0.5 * (lo + hi)
 
-    zlo, zhi = clip_idx(nz, nz)
-    ylo, yhi = clip_idx(ny, ny)
-    xlo, xhi = clip_idx(nx, nx)
-    v = eps_voxels
-    half = 0.5
-    # Ex (nz+1, ny+1, nx): average z then y.
-    az = half * (v[zlo] + v[zhi])
-    ex = half * (az[:, ylo] + az[:, yhi])
-    # Ey (nz+1, ny, nx+1): average z then x.
-    ey = half * (az[:, :, xlo] + az[:, :, xhi])
-    # Ez (nz, ny+1, nx+1): average y then x.
-    ay = half * (v[:, ylo] + v[:, yhi])
-    ez = half * (ay[:, :, xlo] + ay[:, :, xhi])
+    az = pair(eps_voxels, 0)
+    ex = pair(az, 1)  # Ex (nz+1, ny+1, nx): average z then y
+    ey = pair(az, 2)  # Ey (nz+1, ny, nx+1): average z then x
+    ez = pair(pair(eps_voxels, 1), 2)  # Ez (nz, ny+1, nx+1): average y then x
     dto = torch.tensor(np.float32(np.float32(dt) / np.float32(eps0)), device=dev)
     return [dto * (1.0 / ex), dto * (1.0 / ey), dto * (1.0 / ez)]
 

@@ -47,14 +47,18 @@ def shape_class(spec) -> str:
 def heuristic(spec) -> tuple[int, int]:
     """Rules from B200 sweeps of the class step (us per step, best first):
     8-row tiles throughout; 16-plane chunks once the grid holds enough CTAs
-    for many waves (512x512x256: 903 vs 946 with 8), 8-plane chunks below
-    that (192^3: 247 vs 283 with 4), 4-plane chunks for grids of a few
-    million cells, whose CTAs would otherwise not fill the GPU (128^3: 75 vs
-    92 with 8)."""
+    for many waves (512x512x256: 911 vs 952 with 8), 12-plane chunks from 7 M
+    cells (192^3: 240 vs 248 with 8 and 247 with 16, 384x300x256: 428 vs 443 and
+    441, 277x203x150: 269 vs 274), 8-plane chunks below that (192x160x96: 123
+    vs 131 with 4 and 138 with 12), 4-plane chunks for grids of up to 2.5
+    million cells, whose CTAs would otherwise not fill the GPU (128^3: 81 vs 86
+    with 8)."""
     cells = int(np.prod(spec.grid_shape))
     if cells >= 32 * 1024 * 1024:
         return (8, 16)
-    return (8, 8) if cells >= 4 * 1024 * 1024 else (8, 4)
+    if cells >= 7_000_000:
+        return (8, 12)
+    return (8, 8) if cells >= 2_500_000 else (8, 4)
 
 
 def _load(path: str) -> dict:

@@ -1096,18 +1096,22 @@ def dft_change(state: DeviceState, program: DeviceProgram, monitors=None):
     M = len(program.arena.layout)
     r = out.cpu().numpy().reshape(M, 6, -1, 3)
     chosen = range(M) if monitors is None else monitors
-    keys = [(m, ci, f) for m in chosen for ci in range(6) if program.spec.monitors[m].component_mask[ci] > 0
-            for f in range(program.arena.layout[m][1])]
-    finite = all(np.isfinite(r[k][1]) for k in keys)
+    rows = [r[m, np.asarray(program.spec.monitors[m].component_mask) > 0, : program.arena.layout[m][1]].reshape(-1, 3)
+            for m in chosen]
+    rows = np.concatenate(rows) if rows else np.zeros((0, 3))
+    finite = bool(np.isfinite(rows[:, 1]).all())
     if first:
         return None, finite
+    if rows.shape[0] == 0:
+        return 0.0, finite
     tiny = np.finfo(float).tiny
-    changes = []
-    for k in keys:
-        num = float(np.sqrt(r[k][0]))
-        den = max(float(np.sqrt(r[k][1])), float(np.sqrt(r[k][2])))
-        changes.append(0.0 if den <= tiny and num <= tiny else num / den)
-    return max(changes, default=0.0), finite
+    # The largest change as Python's max keeps it: the first value wins over a
+    # later NaN, and a leading NaN stays.
+    with np.errstate(divide="ignore", invalid="ignore"):
+        num, cur, prev = np.sqrt(rows).T
+        den = np.where(prev > cur, prev, cur)
+        change = np.where((den <= tiny) & (num <= tiny), 0.0, num / den)
+    return max(change.tolist()), finite
 
 
 def monitor_values(state: DeviceState, program: DeviceProgram, monitor: int) -> dict:
@@ -1146,7 +1150,8 @@ def _monitor_reduce(state, program, monitor, e, h, scale, weights, profiles=None
     rows = 0 if profiles is None else int(profiles.shape[0])
     dev = program.device
     f64 = lambda a: torch.as_tensor(np.ascontiguousarray(a, np.float64), device=dev)  # noqa: E731
-    keep = [f64(scale), f64(weights)]
+    # No weights: one per point, made where they are read.
+    keep = [f64(scale), torch.ones((2, npts), dtype=torch.float64, device=dev) if weights is None else f64(weights)]
     out = torch.empty((max(rows, 1), nf, 2, 2), dtype=torch.float64, device=dev)
     r = abi.FdtdMonitorReduce()
     r.abi_version = abi.FDTD_ABI_VERSION
@@ -1177,9 +1182,8 @@ def monitor_dft_flux(state: DeviceState, program: DeviceProgram, monitor: int, a
     per_point = iw.size == npts
     if not per_point and measure is None:
         raise ValueError("monitor_dft_flux needs integration weights of one per point or a measure")
-    w = iw if per_point else np.ones(npts)
     sums = _monitor_reduce(state, program, monitor, e, h, _flux_scales(state, program, monitor, base_dt),
-                           np.stack([w, w]))[0]
+                           np.stack([iw, iw]) if per_point else None)[0]
     flux = 0.5 * np.real(sign * (sums[:, 0] - sums[:, 1]))
     return flux if per_point else flux * float(measure)
 
