@@ -41,8 +41,6 @@ namespace {
 
 constexpr int kW = 64;                    // region columns
 constexpr int kGroups = kW / 4;           // threads along x, four columns each
-constexpr int kThreads = 512;
-constexpr int kRows = kThreads / kGroups;  // rows in flight
 constexpr int kMaxT = 16;
 constexpr int kEntryCap = 4096;           // listed gather slots per CTA (more: rescanned each step)
 constexpr int kSmemTwo = 113 * 1024;      // dynamic shared memory that lets two CTAs share an SM
@@ -146,8 +144,10 @@ struct ListEntry {
 
 // Pol 0: TM (Ez, Hx, Hy); 1: TE (Hz, Ex, Ey).  Site: every coefficient is
 // staged per cell; else only the E sources are (E decay and H uniform).
-template <int Pol, bool Cpml, bool Site, bool Metric>
-__global__ void __launch_bounds__(kThreads, 2) block2d_kernel(const __grid_constant__ Block2D q) {
+// kThreads, PerSm: the launch shape (launch_shape below).
+template <int Pol, bool Cpml, bool Site, bool Metric, int kThreads, int PerSm>
+__global__ void __launch_bounds__(kThreads, PerSm) block2d_kernel(const __grid_constant__ Block2D q) {
+  constexpr int kRows = kThreads / kGroups;  // rows in flight
   extern __shared__ __align__(16) float sm[];
   const Step3D& p = q.p;
   const Geo2D& g = q.g;
@@ -824,25 +824,47 @@ bool plan_tiles(const Block2D& q, int pol, bool site, int T, int sms, Plan2D* ou
   return false;
 }
 
-template <int Pol, bool Cpml, bool Site, bool Metric>
-cudaError_t launch_t(cudaStream_t s, const Block2D& q, int ctas, size_t smem) {
-  auto kern = block2d_kernel<Pol, Cpml, Site, Metric>;
+template <int Pol, bool Cpml, bool Site, bool Metric, int Threads, int PerSm>
+cudaError_t launch_s(cudaStream_t s, const Block2D& q, int ctas, size_t smem) {
+  auto kern = block2d_kernel<Pol, Cpml, Site, Metric, Threads, PerSm>;
   const cudaError_t err =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (err != cudaSuccess) return err;
-  kern<<<ctas, kThreads, smem, s>>>(q);
+  kern<<<ctas, Threads, smem, s>>>(q);
   return cudaPeekAtLastError();
 }
 
+// Threads of a CTA: 512, or 768 for tiles of one wave that are taller than the 32
+// rows that 512 threads have in flight.
+int launch_threads(const Geo2D& g, int sms) { return g.gx * g.gy <= sms && g.rows > 512 / kGroups ? 768 : 512; }
+
+// Grids of one wave have an SM to themselves per tile: the steps are then bound
+// by a tile's own instruction chain, and 110 (80) registers a thread shorten it;
+// larger grids run two tiles per SM (us per step, 512 threads two per SM / 512
+// one per SM / 768: 400 x 400 TM 4.67 / 3.90 / 3.66, 200 x 200 3.39 / 2.88 / 3.13,
+// 1000 x 1000 12.4 / 12.6 / 14.1, 3000 x 3000 71 / 90 / 90).
+template <int Pol, bool Cpml, bool Site, bool Metric>
+cudaError_t launch_t(cudaStream_t s, const Block2D& q, int sms, int ctas, size_t smem) {
+  if (q.g.gx * q.g.gy > sms) return launch_s<Pol, Cpml, Site, Metric, 512, 2>(s, q, ctas, smem);
+  if (launch_threads(q.g, sms) == 768) return launch_s<Pol, Cpml, Site, Metric, 768, 1>(s, q, ctas, smem);
+  return launch_s<Pol, Cpml, Site, Metric, 512, 1>(s, q, ctas, smem);
+}
+
 template <int Pol>
-cudaError_t launch_pol(cudaStream_t s, const Block2D& q, bool site, int ctas, size_t smem) {
+cudaError_t launch_pol(cudaStream_t s, const Block2D& q, bool site, int sms, int ctas, size_t smem) {
   const bool metric = has_metric(q.p);
   if (q.p.cpml) {
-    if (metric) return site ? launch_t<Pol, true, true, true>(s, q, ctas, smem) : launch_t<Pol, true, false, true>(s, q, ctas, smem);
-    return site ? launch_t<Pol, true, true, false>(s, q, ctas, smem) : launch_t<Pol, true, false, false>(s, q, ctas, smem);
+    if (metric)
+      return site ? launch_t<Pol, true, true, true>(s, q, sms, ctas, smem)
+                  : launch_t<Pol, true, false, true>(s, q, sms, ctas, smem);
+    return site ? launch_t<Pol, true, true, false>(s, q, sms, ctas, smem)
+                : launch_t<Pol, true, false, false>(s, q, sms, ctas, smem);
   }
-  if (metric) return site ? launch_t<Pol, false, true, true>(s, q, ctas, smem) : launch_t<Pol, false, false, true>(s, q, ctas, smem);
-  return site ? launch_t<Pol, false, true, false>(s, q, ctas, smem) : launch_t<Pol, false, false, false>(s, q, ctas, smem);
+  if (metric)
+    return site ? launch_t<Pol, false, true, true>(s, q, sms, ctas, smem)
+                : launch_t<Pol, false, false, true>(s, q, sms, ctas, smem);
+  return site ? launch_t<Pol, false, true, false>(s, q, sms, ctas, smem)
+              : launch_t<Pol, false, false, false>(s, q, sms, ctas, smem);
 }
 
 }  // namespace
@@ -868,8 +890,6 @@ cudaError_t run_block2d(cudaStream_t s, const Run2D& run, bool* done) {
   cudaError_t err = cudaGetDevice(&device);
   if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (err != cudaSuccess) return err;
-  const int chunks = (q.d.max_points + kThreads - 1) / kThreads;
-  const int nflush = q.samples ? q.d.monitor_count * 3 * chunks : 0;
   int T = std::min(run.steps_per_launch, run.nsteps);
   if (q.samples) T = std::min(T, run.batch / 2);
   T = std::max(1, std::min(T, kMaxT));
@@ -893,17 +913,18 @@ cudaError_t run_block2d(cudaStream_t s, const Run2D& run, bool* done) {
     b.g = plan.g;
     b.g.step_offset = at;
     b.g.slot0 = (n & 1) * (run.batch / 2);
-    b.g.nflush = n > 0 ? nflush : 0;
+    const int threads = launch_threads(b.g, sms);
+    b.g.nflush = n > 0 && q.samples ? q.d.monitor_count * 3 * ((q.d.max_points + threads - 1) / threads) : 0;
     b.g.flush_first = at - prev;
     b.g.flush_count = prev;
     b.g.flush_slot0 = ((n + 1) & 1) * (run.batch / 2);
     const int ctas = b.g.nflush + b.g.gx * b.g.gy;
-    err = pol == 0 ? launch_pol<0>(s, b, site, ctas, plan.smem) : launch_pol<1>(s, b, site, ctas, plan.smem);
+    err = pol == 0 ? launch_pol<0>(s, b, site, sms, ctas, plan.smem) : launch_pol<1>(s, b, site, sms, ctas, plan.smem);
     if (err != cudaSuccess) return err;
     at += count;
     prev = count;
   }
-  if (q.samples && nflush > 0) {
+  if (q.samples) {
     const dim3 grid((q.d.max_points + 255) / 256, q.d.monitor_count * 3, 1);
     flush_raw_kernel<<<grid, 256, 0, s>>>(q.d, q.samples, q.counter, at - prev,
                                           ((launches - 1) & 1) * (run.batch / 2), prev, pol);
