@@ -766,10 +766,14 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
         const bool AX = SX && (!RT || shell_x), AY = SY && (!RT || shell_y), AZ = SZ && (!RT || shell_z);
         const bool at_x0 = FC && xface, at_y0 = FC && yface;
         const int jh = j0 - 1, ih = i0 - 1;  // the halo row and column
-        // Which warps recompute a halo this plane (never on a pre-plane).
-        const bool halo_row_x = emit && warp == 0 && !at_y0;              // Hx on row j0-1
-        const bool halo_row_z = emit && warp == 1 && !at_y0;              // Hz on row j0-1
-        const bool halo_col = emit && warp == 2 && lane < TY && !at_x0;   // Hy, Hz on column i0-1
+        // Which warps recompute a halo this plane (never on a pre-plane): see there.
+        constexpr int kColY = 2, kColZ = NW == 8 ? 5 : 3;
+        [[maybe_unused]] const bool halo_rows = emit && !at_y0;                                 // Hx, Hz on row j0-1
+        [[maybe_unused]] const bool halo_col_y = emit && warp == kColY && lane < TY && !at_x0;  // Hy on column i0-1
+        [[maybe_unused]] const bool halo_col_z = emit && warp == kColZ && lane < TY && !at_x0;  // Hz on column i0-1
+        [[maybe_unused]] const bool halo_row_x = emit && warp == 0 && !at_y0;              // Hx on row j0-1
+        [[maybe_unused]] const bool halo_row_z = emit && warp == 1 && !at_y0;              // Hz on row j0-1
+        [[maybe_unused]] const bool halo_col = emit && warp == 2 && lane < TY && !at_x0;   // Hy, Hz on column i0-1
         const int jc = j0 + lane;                                         // halo_col's row
         // ---- every global load of the plane goes out first ----
         // psi of the H terms: own cells and halos.
@@ -872,74 +876,150 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
             for (int n = 0; n < 3; ++n) copy16(&sm.h[hs][n][rc], p.site_c[n] + o);
           }
         }
-        // ---- recomputed halo: row j0-1 (Hx by warp 0, Hz by warp 1) and
-        //      column i0-1 (Hy, Hz by warp 2), read-only on psi ----
-        if (halo_row_x && !zZ) {
-          const int b = c0;
-          float4 qa, qb;
-          if (AY) qa = psi4_fetch<1>(p.ht[0], slot_of(p.ht[0], jh), k, jh, i, nvv);
-          if (AZ) qb = psi4_fetch<0>(p.ht[1], slot_of(p.ht[1], k), k, jh, i, nvv);
-          float4 d0 = MH4(sub4(ld4(E0z + b + BX), ld4(E0z + b)), 1, jh), d1 = MH4(sub4(ld4(E1y + b), ld4(E0y + b)), 0, k);
-          if (AY) d0 = psi4_apply<Exact, 1>(p.ht[0], sm.cc[0], slot_of(p.ht[0], jh), qa, k, jh, i, res, d0, false, nvv);
-          if (AZ) d1 = psi4_apply<Exact, 0>(p.ht[1], sm.cc[1], slot_of(p.ht[1], k), qb, k, jh, i, res, d1, false, nvv);
-          float4 h;
-          if constexpr (Lossy)
-            h = h4_loss<Exact>(ld4(HOx + b), sm.hcls, *reinterpret_cast<const uint32_t*>(HIDS + 16 + 4 * lane), 0,
-                               d0, d1);
-          else
-            h = h4<Exact>(ld4(HOx + b), sm.hcoef[0], sm.hcoef[3], d0, d1);
-          if (at_x0 && lane == 0 && wx0) h.x = 0.0f;
-          st4(&sm.hn[0][0][b], h);
-        } else if (halo_row_z) {
-          const int b = c0;
-          float4 qa, qb;
-          const int xs4 = AX ? sm.xst[1][lane] : 0;
-          if (AX) {
-            if (xstage) {  // row j0-1 of the staged Hzx box (cells outside the slab are not read)
-              const float* q = &sm.xps[hs][1][(xs4 >> 4) - sm.xwin[1]];
-              qa = make_float4(q[0], q[1], q[2], q[3]);
-            } else {
-              qa = psix_fetch(p.ht[4], xs4, k, jh);
+        // ---- recomputed halo of row j0-1 (Hx, Hz) and column i0-1 (Hy, Hz),
+        //      read-only on psi.  Full tiles: the row as vectors, Hx by warp 0 and Hz
+        //      by warp 1, the column by warp 2.  Partial grids, whose last tile column
+        //      always runs the run-time body: every warp takes 16 columns of the row
+        //      (8-warp tiles) as scalars, Hx on lanes 0-15 and Hz on 16-31, and two
+        //      warps a component of the column each, so that no warp brings a second
+        //      H update to the plane's barrier (us per step, vectors / spread:
+        //      277 x 203 x 150 268 / 247, 192^3 240 / 227; full tiles 512 x 512 x 256
+        //      909 / 924, 256 x 192 x 128 rectilinear 148 / 151). ----
+        if constexpr (Partial) {
+          if (halo_rows) {
+#pragma unroll
+            for (int q = 0; q < 8 / NW; ++q) {
+              const bool isz = lane >= 16;
+              const int xo = (TX / NW) * warp + 16 * q + (lane & 15), x = i0 + xo, b = 4 + xo;
+              const float* E0 = isz ? E0y : E0z;
+              const float* Ea = isz ? E0x : E0y;
+              const float* Eb = isz ? E0x + BX : E1y;
+              float d0 = E0[b + (isz ? 1 : BX)] - E0[b], d1 = Eb[b] - Ea[b];  // Hx: dEz/dy, dEy/dz; Hz: dEy/dx, dEx/dy
+              if constexpr (Metric) {
+                const float my = p.metric_h[1][clampi(jh, Y - 1)];
+                d0 = d0 * (isz ? p.metric_h[2][clampi(x, X - 1)] : my);
+                d1 = d1 * (isz ? my : p.metric_h[0][clampi(k, Z - 1)]);
+              } else {
+                d0 = D1(d0);
+                d1 = D1(d1);
+              }
+              if ((SX || SY || SZ) && x < X) {
+                if (!isz) {
+                  if (AY && !zZ) d0 = psi1_apply<Exact, 1>(p.ht[0], sm.cc[0], psi1_fetch<1>(p.ht[0], k, jh, x), k, jh, x, res, d0, false);
+                  if (AZ && !zZ) d1 = psi1_apply<Exact, 0>(p.ht[1], sm.cc[1], psi1_fetch<0>(p.ht[1], k, jh, x), k, jh, x, res, d1, false);
+                } else {
+                  if (AX) {
+                    const int slot = slot_of(p.ht[4], x);
+                    if (slot >= 0) {
+                      const float psi = xstage ? sm.xps[hs][1][slot - sm.xwin[1]] : p.ht[4].psi_in[psi_off<2>(p.ht[4], slot, k, jh, x)];
+                      float unused;
+                      d0 = cpml_d<Exact>(sm.cc[4][slot], res, psi, d0, &unused);
+                    }
+                  }
+                  if (AY) d1 = psi1_apply<Exact, 1>(p.ht[5], sm.cc[5], psi1_fetch<1>(p.ht[5], k, jh, x), k, jh, x, res, d1, false);
+                }
+              }
+              const int n = isz ? 2 : 0;
+              float2 c;
+              if constexpr (Lossy) c = sm.hcls[(HIDS[16 + xo] & kHClassMask) * 4 + n];
+              else c = make_float2(sm.hcoef[n], sm.hcoef[3 + n]);
+              float h = h1<Exact>(sm.h[hs][n][b], c.x, c.y, d0, d1);
+              if (isz ? ((z0 && wz0) || (zZ && wz1)) : (at_x0 && xo == 0 && wx0)) h = 0.0f;
+              sm.hn[n][0][b] = h;
             }
           }
-          if (AY) qb = psi4_fetch<1>(p.ht[5], slot_of(p.ht[5], jh), k, jh, i, nvv);
-          const float4 eyh = ld4(E0y + b);
-          float e4 = __shfl_down_sync(kFull, eyh.x, 1);
-          if (lane == 31) e4 = E0y[b + 4];
-          float4 d0 = MH4x(sub4(next4(eyh, e4), eyh), i), d1 = MH4(sub4(ld4(E0x + b + BX), ld4(E0x + b)), 1, jh);
-          if (AX) d0 = psix_apply<Exact>(p.ht[4], sm.cc[4], xs4, qa, k, jh, res, d0, false);
-          if (AY) d1 = psi4_apply<Exact, 1>(p.ht[5], sm.cc[5], slot_of(p.ht[5], jh), qb, k, jh, i, res, d1, false, nvv);
-          float4 h;
-          if constexpr (Lossy)
-            h = h4_loss<Exact>(ld4(HOz + b), sm.hcls, *reinterpret_cast<const uint32_t*>(HIDS + 16 + 4 * lane), 2, d0,
-                               d1);
-          else
-            h = h4<Exact>(ld4(HOz + b), sm.hcoef[2], sm.hcoef[5], d0, d1);
-          if ((z0 && wz0) || (zZ && wz1)) h = make_float4(0.f, 0.f, 0.f, 0.f);
-          st4(&sm.hn[2][0][b], h);
-        } else if (halo_col) {
-          const int rr = 1 + lane, b = rr * BX + 3;
-          const bool hz_ok = !(lyr && jc == Y);  // Hz has no row Y
-          float qc0 = 0.f, qc1 = 0.f, qc2 = 0.f, qc3 = 0.f;
-          if (AZ && !zZ) qc0 = psi1_fetch<0>(p.ht[2], k, jc, ih);
-          if (AX && !zZ) qc1 = psi1_fetch<2>(p.ht[3], k, jc, ih);
-          if (AX && hz_ok) qc2 = psi1_fetch<2>(p.ht[4], k, jc, ih);
-          if (AY && hz_ok) qc3 = psi1_fetch<1>(p.ht[5], k, jc, ih);
-          float d0 = MH(E1x[b] - E0x[b], 0, k), d1 = MH(E0z[b + 1] - E0z[b], 2, ih);  // Hy: dEx/dz, dEz/dx
-          if (AZ && !zZ) d0 = psi1_apply<Exact, 0>(p.ht[2], sm.cc[2], qc0, k, jc, ih, res, d0, false);
-          if (AX) d1 = psi1_apply<Exact, 2>(p.ht[3], sm.cc[3], qc1, k, jc, ih, res, d1, false);
-          const int hc = Lossy ? (HIDS[rr * T::HW + 15] & kHClassMask) : 0;  // the halo column's H class
-          const float2 cy = Lossy ? sm.hcls[hc * 4 + 1] : make_float2(sm.hcoef[1], sm.hcoef[4]);
-          const float2 cz = Lossy ? sm.hcls[hc * 4 + 2] : make_float2(sm.hcoef[2], sm.hcoef[5]);
-          float hyv = h1<Exact>(HOy[b], cy.x, cy.y, d0, d1);
-          if ((at_y0 && jc == 0 && wy0) || (lyr && jc == Y && wy1)) hyv = 0.0f;
-          float f0 = MH(E0y[b + 1] - E0y[b], 2, ih), f1 = MH(E0x[b + BX] - E0x[b], 1, jc);  // Hz: dEy/dx, dEx/dy
-          if (AX && hz_ok) f0 = psi1_apply<Exact, 2>(p.ht[4], sm.cc[4], qc2, k, jc, ih, res, f0, false);
-          if (AY && hz_ok) f1 = psi1_apply<Exact, 1>(p.ht[5], sm.cc[5], qc3, k, jc, ih, res, f1, false);
-          sm.hn[1][rr][3] = hyv;
-          float hzv = h1<Exact>(HOz[b], cz.x, cz.y, f0, f1);
-          if ((z0 && wz0) || (zZ && wz1)) hzv = 0.0f;
-          sm.hn[2][rr][3] = hzv;
+          if (halo_col_y) {
+            const int rr = 1 + lane, b = rr * BX + 3;
+            float d0 = MH(E1x[b] - E0x[b], 0, k), d1 = MH(E0z[b + 1] - E0z[b], 2, ih);  // Hy: dEx/dz, dEz/dx
+            if (AZ && !zZ) d0 = psi1_apply<Exact, 0>(p.ht[2], sm.cc[2], psi1_fetch<0>(p.ht[2], k, jc, ih), k, jc, ih, res, d0, false);
+            if (AX && !zZ) d1 = psi1_apply<Exact, 2>(p.ht[3], sm.cc[3], psi1_fetch<2>(p.ht[3], k, jc, ih), k, jc, ih, res, d1, false);
+            float2 c;  // the halo column's H class, or the uniform coefficients
+            if constexpr (Lossy) c = sm.hcls[(HIDS[rr * T::HW + 15] & kHClassMask) * 4 + 1];
+            else c = make_float2(sm.hcoef[1], sm.hcoef[4]);
+            float hyv = h1<Exact>(HOy[b], c.x, c.y, d0, d1);
+            if ((at_y0 && jc == 0 && wy0) || (lyr && jc == Y && wy1)) hyv = 0.0f;
+            sm.hn[1][rr][3] = hyv;
+          } else if (halo_col_z) {
+            const int rr = 1 + lane, b = rr * BX + 3;
+            const bool hz_ok = !(lyr && jc == Y);  // Hz has no row Y
+            float f0 = MH(E0y[b + 1] - E0y[b], 2, ih), f1 = MH(E0x[b + BX] - E0x[b], 1, jc);  // Hz: dEy/dx, dEx/dy
+            if (AX && hz_ok) f0 = psi1_apply<Exact, 2>(p.ht[4], sm.cc[4], psi1_fetch<2>(p.ht[4], k, jc, ih), k, jc, ih, res, f0, false);
+            if (AY && hz_ok) f1 = psi1_apply<Exact, 1>(p.ht[5], sm.cc[5], psi1_fetch<1>(p.ht[5], k, jc, ih), k, jc, ih, res, f1, false);
+            float2 c;
+            if constexpr (Lossy) c = sm.hcls[(HIDS[rr * T::HW + 15] & kHClassMask) * 4 + 2];
+            else c = make_float2(sm.hcoef[2], sm.hcoef[5]);
+            float hzv = h1<Exact>(HOz[b], c.x, c.y, f0, f1);
+            if ((z0 && wz0) || (zZ && wz1)) hzv = 0.0f;
+            sm.hn[2][rr][3] = hzv;
+          }
+        } else {
+          if (halo_row_x && !zZ) {
+            const int b = c0;
+            float4 qa, qb;
+            if (AY) qa = psi4_fetch<1>(p.ht[0], slot_of(p.ht[0], jh), k, jh, i, nvv);
+            if (AZ) qb = psi4_fetch<0>(p.ht[1], slot_of(p.ht[1], k), k, jh, i, nvv);
+            float4 d0 = MH4(sub4(ld4(E0z + b + BX), ld4(E0z + b)), 1, jh), d1 = MH4(sub4(ld4(E1y + b), ld4(E0y + b)), 0, k);
+            if (AY) d0 = psi4_apply<Exact, 1>(p.ht[0], sm.cc[0], slot_of(p.ht[0], jh), qa, k, jh, i, res, d0, false, nvv);
+            if (AZ) d1 = psi4_apply<Exact, 0>(p.ht[1], sm.cc[1], slot_of(p.ht[1], k), qb, k, jh, i, res, d1, false, nvv);
+            float4 h;
+            if constexpr (Lossy)
+              h = h4_loss<Exact>(ld4(HOx + b), sm.hcls, *reinterpret_cast<const uint32_t*>(HIDS + 16 + 4 * lane), 0,
+                                 d0, d1);
+            else
+              h = h4<Exact>(ld4(HOx + b), sm.hcoef[0], sm.hcoef[3], d0, d1);
+            if (at_x0 && lane == 0 && wx0) h.x = 0.0f;
+            st4(&sm.hn[0][0][b], h);
+          } else if (halo_row_z) {
+            const int b = c0;
+            float4 qa, qb;
+            const int xs4 = AX ? sm.xst[1][lane] : 0;
+            if (AX) {
+              if (xstage) {  // row j0-1 of the staged Hzx box (cells outside the slab are not read)
+                const float* q = &sm.xps[hs][1][(xs4 >> 4) - sm.xwin[1]];
+                qa = make_float4(q[0], q[1], q[2], q[3]);
+              } else {
+                qa = psix_fetch(p.ht[4], xs4, k, jh);
+              }
+            }
+            if (AY) qb = psi4_fetch<1>(p.ht[5], slot_of(p.ht[5], jh), k, jh, i, nvv);
+            const float4 eyh = ld4(E0y + b);
+            float e4 = __shfl_down_sync(kFull, eyh.x, 1);
+            if (lane == 31) e4 = E0y[b + 4];
+            float4 d0 = MH4x(sub4(next4(eyh, e4), eyh), i), d1 = MH4(sub4(ld4(E0x + b + BX), ld4(E0x + b)), 1, jh);
+            if (AX) d0 = psix_apply<Exact>(p.ht[4], sm.cc[4], xs4, qa, k, jh, res, d0, false);
+            if (AY) d1 = psi4_apply<Exact, 1>(p.ht[5], sm.cc[5], slot_of(p.ht[5], jh), qb, k, jh, i, res, d1, false, nvv);
+            float4 h;
+            if constexpr (Lossy)
+              h = h4_loss<Exact>(ld4(HOz + b), sm.hcls, *reinterpret_cast<const uint32_t*>(HIDS + 16 + 4 * lane), 2, d0,
+                                 d1);
+            else
+              h = h4<Exact>(ld4(HOz + b), sm.hcoef[2], sm.hcoef[5], d0, d1);
+            if ((z0 && wz0) || (zZ && wz1)) h = make_float4(0.f, 0.f, 0.f, 0.f);
+            st4(&sm.hn[2][0][b], h);
+          } else if (halo_col) {
+            const int rr = 1 + lane, b = rr * BX + 3;
+            const bool hz_ok = !(lyr && jc == Y);  // Hz has no row Y
+            float qc0 = 0.f, qc1 = 0.f, qc2 = 0.f, qc3 = 0.f;
+            if (AZ && !zZ) qc0 = psi1_fetch<0>(p.ht[2], k, jc, ih);
+            if (AX && !zZ) qc1 = psi1_fetch<2>(p.ht[3], k, jc, ih);
+            if (AX && hz_ok) qc2 = psi1_fetch<2>(p.ht[4], k, jc, ih);
+            if (AY && hz_ok) qc3 = psi1_fetch<1>(p.ht[5], k, jc, ih);
+            float d0 = MH(E1x[b] - E0x[b], 0, k), d1 = MH(E0z[b + 1] - E0z[b], 2, ih);  // Hy: dEx/dz, dEz/dx
+            if (AZ && !zZ) d0 = psi1_apply<Exact, 0>(p.ht[2], sm.cc[2], qc0, k, jc, ih, res, d0, false);
+            if (AX) d1 = psi1_apply<Exact, 2>(p.ht[3], sm.cc[3], qc1, k, jc, ih, res, d1, false);
+            const int hc = Lossy ? (HIDS[rr * T::HW + 15] & kHClassMask) : 0;  // the halo column's H class
+            const float2 cy = Lossy ? sm.hcls[hc * 4 + 1] : make_float2(sm.hcoef[1], sm.hcoef[4]);
+            const float2 cz = Lossy ? sm.hcls[hc * 4 + 2] : make_float2(sm.hcoef[2], sm.hcoef[5]);
+            float hyv = h1<Exact>(HOy[b], cy.x, cy.y, d0, d1);
+            if ((at_y0 && jc == 0 && wy0) || (lyr && jc == Y && wy1)) hyv = 0.0f;
+            float f0 = MH(E0y[b + 1] - E0y[b], 2, ih), f1 = MH(E0x[b + BX] - E0x[b], 1, jc);  // Hz: dEy/dx, dEx/dy
+            if (AX && hz_ok) f0 = psi1_apply<Exact, 2>(p.ht[4], sm.cc[4], qc2, k, jc, ih, res, f0, false);
+            if (AY && hz_ok) f1 = psi1_apply<Exact, 1>(p.ht[5], sm.cc[5], qc3, k, jc, ih, res, f1, false);
+            sm.hn[1][rr][3] = hyv;
+            float hzv = h1<Exact>(HOz[b], cz.x, cz.y, f0, f1);
+            if ((z0 && wz0) || (zZ && wz1)) hzv = 0.0f;
+            sm.hn[2][rr][3] = hzv;
+          }
         }
         __syncthreads();
         if (!emit) {
@@ -1014,7 +1094,7 @@ __global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 4)
           fz0 = xtake(fz0, sm.xst[3][lane], sm.xd[1][warp]);
         }
         const float4 ex = ld4(E0x + rc), ey = ld4(E0y + rc), ez = ld4(E0z + rc);  // E(k) of the own cells
-        const uint32_t w4 = Site ? 0u : *reinterpret_cast<const uint32_t*>(IDS + warp * TX + 4 * lane);
+        [[maybe_unused]] const uint32_t w4 = Site ? 0u : *reinterpret_cast<const uint32_t*>(IDS + warp * TX + 4 * lane);
         float4 nx, ny, nz;
         if constexpr (Lossy) {
           const float2* ec = reinterpret_cast<const float2*>(sm.cls);
