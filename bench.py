@@ -486,6 +486,10 @@ def main():
     chunks = [min(R.GRAPH_CHUNK_STEPS, args.steps - c) for c in range(0, args.steps, R.GRAPH_CHUNK_STEPS)]
     flushes = sum(-(-n // prog.dft_batch) for n in chunks) if spec.monitors and prog.dft_batch > 1 else 0
     launches = per_step * args.steps + flushes + len(chunks)
+    if spec.ndim == 2:  # up to eight steps per launch, the launches of the steps' parity; a last flush; the counters
+        most = min(8, prog.dft_batch // 2) if spec.monitors else 8
+        blocks = [-(-n // max(1, most)) for n in chunks]
+        launches = sum(b + ((b ^ n) & 1) for b, n in zip(blocks, chunks)) + len(chunks) * (2 if spec.monitors else 1)
 
     # ---- dominant kernel alone: the fused step without sources or monitors ---
     if args.scene == "3d_512":
