@@ -45,6 +45,7 @@ constexpr int kMaxT = 16;
 constexpr int kEntryCap = 4096;           // listed gather slots per CTA (more: rescanned each step)
 constexpr int kSmemTwo = 113 * 1024;      // dynamic shared memory that lets two CTAs share an SM
 constexpr int kStatic = 2048;             // room for the static shared memory
+constexpr int kSmemMax = kSmemTwo - kStatic;  // most dynamic shared memory of any plan
 
 struct Geo2D {
   int T, TX, TY, rows, gx, gy;
@@ -813,7 +814,7 @@ bool plan_tiles(const Block2D& q, int pol, bool site, int T, int sms, Plan2D* ou
     g.dft_cap = q.samples ? std::min(kEntryCap, g.TY * g.TX) : 0;
     g.o_list = take(4 * g.rec_cap + 2 * g.dft_cap);
     const size_t bytes = std::max(static_cast<size_t>(at) * 4, sizeof(FlushShared));
-    if (bytes + kStatic > kSmemTwo) {
+    if (bytes > kSmemMax) {
       if (g.TY == 8) return false;
       continue;
     }
@@ -827,8 +828,9 @@ bool plan_tiles(const Block2D& q, int pol, bool site, int T, int sms, Plan2D* ou
 template <int Pol, bool Cpml, bool Site, bool Metric, int Threads, int PerSm>
 cudaError_t launch_s(cudaStream_t s, const Block2D& q, int ctas, size_t smem) {
   auto kern = block2d_kernel<Pol, Cpml, Site, Metric, Threads, PerSm>;
-  const cudaError_t err =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  // The limit belongs to the function, not to the launch: every thread sets the
+  // same one, so that none lowers it between another's setting and its launch.
+  const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
   if (err != cudaSuccess) return err;
   kern<<<ctas, Threads, smem, s>>>(q);
   return cudaPeekAtLastError();
