@@ -16,7 +16,7 @@ import threading
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "_fdtd_b200.so")
 
-FDTD_ABI_VERSION = 14
+FDTD_ABI_VERSION = 15
 FDTD_F32, FDTD_S32, FDTD_BF16, FDTD_U8, FDTD_F64 = 0, 1, 2, 3, 4
 FDTD_FLAG_GRAPH_CACHE = 1 << 7
 FDTD_FLAG_DFT_OVERLAP = 1 << 16
@@ -128,6 +128,8 @@ class FdtdDft(ctypes.Structure):
         ("weight_sum", FdtdBuffer),
         ("samples", FdtdBuffer),
         ("affine", FdtdBuffer),
+        ("slot_order", FdtdBuffer),
+        ("slot_first", FdtdBuffer),
     ]
 
 
@@ -210,6 +212,8 @@ class FdtdRecorder(ctypes.Structure):
         ("times", FdtdBuffer),
         ("count", FdtdBuffer),
         ("box", (ctypes.c_int32 * 4) * 6),
+        ("order", FdtdBuffer * 6),
+        ("first", FdtdBuffer * 6),
     ]
 
 

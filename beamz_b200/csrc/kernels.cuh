@@ -184,6 +184,14 @@ struct DftDev {
   const int* affine;  // [M, 6, 24] affine plans (FdtdDft::affine), or null
 };
 
+// Gather slots sorted by the cell they read (FdtdDft::slot_order / slot_first).
+constexpr int kSlotBlock = 16;  // columns per entry of `first`
+struct SlotOrder {
+  const int* order = nullptr;
+  const int* first = nullptr;
+  int n = 0;
+};
+
 // Monitor-plane reduction (analysis.cu); see FdtdMonitorReduce.
 struct MonitorReduceDev {
   const float* re = nullptr;
@@ -209,6 +217,7 @@ struct RecorderDev {
   struct Box {                                // 2D: the plan is this box of cells, row by row, weight 1
     int y0 = 0, x0 = 0, ny = 0, nx = 0;       // ny = 0: it is not
   } box[6];
+  SlotOrder order[6];                         // 2D: the values by cell (those without one last)
   const int* idx[6] = {};
   const float* w[6] = {};
   float* values[6] = {};
@@ -235,6 +244,7 @@ struct Run2D {
   Step3D bank[2];
   int* counter = nullptr;
   DftDev dft{};
+  SlotOrder slots;  // the DFT gather slots, by active component and cell
   float* samples = nullptr;
   int batch = 0;
   int nsrc = 0;

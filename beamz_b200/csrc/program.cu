@@ -88,6 +88,17 @@ bool has_metric(const FdtdProgram& p) {
   return false;
 }
 
+// Gather slots by cell (FdtdDft::slot_order, FdtdRecorder::order): absent, or of
+// the declared sizes.
+bool slot_order_ok(const FdtdProgram& p, const Layout& L, const FdtdBuffer& order, const FdtdBuffer& first, int comps,
+                   int64_t most) {
+  if (order.data == nullptr && first.data == nullptr) return true;
+  if (p.ndim != 2 || order.data == nullptr || first.data == nullptr) return false;
+  const int64_t blocks = (L.X + kSlotBlock) / kSlotBlock;  // of X + 1 columns
+  return order.element_type == FDTD_S32 && first.element_type == FDTD_S32 && elements(order) >= 0 &&
+         elements(order) <= most && elements(first) == comps * (L.Y + 1) * (blocks + 1);
+}
+
 int validate(const FdtdProgram& p) {
   if (p.abi_version != FDTD_ABI_VERSION) return kInvalid;
   Layout L;
@@ -269,6 +280,7 @@ int validate(const FdtdProgram& p) {
         (!is_f32(d.samples) || (elements(d.samples) != d.batch * per_step &&
                                 (p.ndim != 2 || elements(d.samples) != d.batch * per_step * d.indices.dims[2]))))
       return kInvalid;
+    if (!slot_order_ok(p, L, d.slot_order, d.slot_first, 3, elements(d.indices))) return kInvalid;
   }
   if (p.recorder_count < 0 || p.recorder_count > FDTD_MAX_RECORDERS) return kInvalid;
   if (p.recorder_count > 0 && (!is_f32(p.step_time) || elements(p.step_time) < 1 || p.step_time.data == nullptr))
@@ -301,12 +313,22 @@ int validate(const FdtdProgram& p) {
               box[1] + box[3] > cd.x || static_cast<int64_t>(box[2]) * box[3] != V)
             return kInvalid;
         }
+        if (!slot_order_ok(p, L, rec.order[q], rec.first[q], 1, V)) return kInvalid;
+        if (rec.order[q].data != nullptr && elements(rec.order[q]) != V) return kInvalid;
       }
       if (!is_f32(rec.values[q]) || elements(rec.values[q]) != cap * V || (cap * V > 0 && rec.values[q].data == nullptr))
         return kInvalid;
     }
   }
   return 0;
+}
+
+SlotOrder slot_order(const FdtdBuffer& order, const FdtdBuffer& first) {
+  SlotOrder s;
+  s.order = static_cast<const int*>(order.data);
+  s.first = static_cast<const int*>(first.data);
+  s.n = order.data ? static_cast<int>(elements(order)) : 0;
+  return s;
 }
 
 // Device view of recorder r reading the component arrays of `bank`.
@@ -337,6 +359,7 @@ RecorderDev recorder_dev(const FdtdProgram& p, const Layout& L, int r, const Fdt
       d.w[q] = static_cast<const float*>(rec.weights[q].data);
       V = rec.indices[q].dims[1];
       d.box[q] = {rec.box[q][0], rec.box[q][1], rec.box[q][2], rec.box[q][3]};
+      d.order[q] = slot_order(rec.order[q], rec.first[q]);
     }
     d.values[q] = static_cast<float*>(rec.values[q].data);
     d.start[q + 1] = d.start[q] + V;
@@ -619,7 +642,8 @@ bool wants_side_stream(const FdtdProgram& p) {
 // A 2D program's steps, several per launch (block2d.cu): fused programs whose
 // CPML memories are all double-banked, whose monitors are batched with a raw
 // sample ring (one gather slot per point, or samples sized for every slot) and
-// whose recorders read single cells.  *done stays false for the others.
+// whose recorders read single cells, with the slots of both sorted by cell.
+// *done stays false for the others.
 cudaError_t enqueue_block2d(cudaStream_t s, const FdtdProgram& p, const Layout& L, bool* done) {
   *done = false;
   if (p.ndim != 2 || p.schedule != FDTD_SCHEDULE_FUSED || p.material_kind != FDTD_MATERIAL_SITE || p.nsteps < 1)
@@ -630,15 +654,19 @@ cudaError_t enqueue_block2d(cudaStream_t s, const FdtdProgram& p, const Layout& 
     const FdtdDft& d = p.dft;
     if (d.batch < 2 || d.samples.data == nullptr || d.indices.dims[3] < 1 || d.freqs.dims[1] > 64) return cudaSuccess;
     if (elements(d.samples) != static_cast<int64_t>(d.batch) * elements(d.indices)) return cudaSuccess;
-    if (elements(d.indices) >= (int64_t{1} << 31)) return cudaSuccess;
+    if (elements(d.indices) >= (int64_t{1} << 31) || d.slot_order.data == nullptr) return cudaSuccess;
     run.dft = make_dft(p, p.fields);
+    run.slots = slot_order(d.slot_order, d.slot_first);
     run.samples = static_cast<float*>(d.samples.data);
     run.batch = d.batch;
   }
   for (int r = 0; r < p.recorder_count; ++r) {
     run.rec[r] = recorder_dev(p, L, r, p.fields);
-    for (int q = 0; q < run.rec[r].ncomp; ++q)
-      if (run.rec[r].slots[q] > 1 || run.rec[r].start[q + 1] >= (int64_t{1} << 31)) return cudaSuccess;
+    const RecorderDev& rec = run.rec[r];
+    for (int q = 0; q < rec.ncomp; ++q) {
+      if (rec.slots[q] > 1 || rec.start[q + 1] >= (int64_t{1} << 31)) return cudaSuccess;
+      if (rec.slots[q] == 1 && rec.box[q].ny == 0 && rec.order[q].order == nullptr) return cudaSuccess;
+    }
   }
   run.nrec = p.recorder_count;
   run.pol = p.polarization;

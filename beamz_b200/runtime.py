@@ -405,6 +405,58 @@ def _affine_plan(idx, w):
             + [int(v) for v in bits] + [0] * (8 - k))
 
 
+def _slots_by_cell(cells, live, widths, rows: int, cols: int):
+    """Gather slots sorted by the cell they read (FdtdDft.slot_order): positions
+    in the flattened ``cells`` [components, n], live ones first by component, row
+    and column, and per component, row and 16-column block of a rows x cols
+    lattice the number of slots before it.  ``widths``: row length of each
+    component."""
+    torch = _torch()
+    dev = cells.device
+    blocks = -(-cols // 16)
+    group = torch.arange(cells.shape[0] * rows, device=dev).view(-1, rows, 1)
+    width = torch.tensor(widths, device=dev).view(-1, 1)
+    key = (torch.div(cells, width, rounding_mode="floor") + group[:, 0]) * (16 * blocks) + cells % width
+    key = torch.where(live, key, group.numel() * 16 * blocks).reshape(-1)
+    key, order = torch.sort(key)
+    first = torch.searchsorted(key, group * (16 * blocks) + 16 * torch.arange(blocks + 1, device=dev))
+    return order, first.to(torch.int32)
+
+
+def slot_samples_fit(monitors: int, slots: int, points: int, batch: int = 16) -> bool:
+    """Does a 2D program buffer every gather slot's value (FdtdDft.samples
+    [batch, M, 6, K, P], for several steps per launch)?  Up to 1 GiB with one slot
+    per point, as many bytes as the interpolated samples take; with more slots up
+    to 128 MiB, about the L2: a whole-plane monitor of four slots per point takes
+    10.8 us per step against 19 in single steps at 200 x 200 (61 MB), but 25.3
+    against 23.9 at 400 x 400 (245 MB)."""
+    return batch >= 2 and 4 * batch * monitors * 6 * slots * points <= (1 << 30 if slots == 1 else 1 << 27)
+
+
+def _dft_slots(arena, components, shapes, lattice):
+    """FdtdDft.slot_order and slot_first of a 2D program's packed plan."""
+    torch = _torch()
+    M, _six, K, P = (int(v) for v in arena.indices.shape)
+    n = len(components)
+    at = torch.arange(arena.indices.numel(), device=arena.indices.device).view(M, 6, K, P)[:, components]
+    cells = arena.indices[:, components].long()
+    size = torch.tensor([int(np.prod(shapes[c])) for c in components], device=cells.device).view(1, n, 1, 1)
+    live = (arena.weights[:, components] != 0).cumprod(dim=2).bool()  # a zero weight ends a point's gather
+    live &= (cells >= 0) & (cells < size) & (arena.masks[:, components] != 0).view(M, n, 1, 1)
+    live &= torch.arange(P, device=cells.device) < arena.counts[:, 1].view(M, 1, 1, 1)
+    flat = lambda t: t.transpose(0, 1).reshape(n, -1)  # noqa: E731
+    order, first = _slots_by_cell(flat(cells), flat(live), [int(shapes[c][1]) for c in components], *lattice)
+    return flat(at).reshape(-1)[order].to(torch.int32), first
+
+
+def _recorder_slots(indices, weights, shape, lattice):
+    """FdtdRecorder.order and first of one packed one-slot plan of a 2D program."""
+    cells = indices.long()
+    live = (weights != 0) & (cells >= 0) & (cells < int(np.prod(shape)))
+    order, first = _slots_by_cell(cells, live, [int(shape[1])], *lattice)
+    return order.to(indices.dtype), first
+
+
 def _pack_plan(lib, stream, indices, weights, dims, strides, device):
     """One (V, K) gather plan as device [K, V] arrays in the device layout,
     nonzero weights first per value (fdtd_pack_gather)."""
@@ -701,12 +753,21 @@ class DeviceProgram:
                 s.metric_h[a] = buf(_f32(spec.metrics.along(f"e_to_h_{name}", n), dev))
                 s.metric_e[a] = buf(_f32(spec.metrics.along(f"h_to_e_{name}", n + 1), dev))
         # Monitors.
+        lattice = tuple(int(v) + 1 for v in spec.grid_shape)
         self.arena = pack_dft_monitors(spec.monitors, dev, [self.shapes[c] for c in COMPONENTS], self._strides)
+        self.slot_samples = False  # are every gather slot's values buffered (2D, several steps per launch)?
         if self.arena is not None:
             a = self.arena
             s.dft.monitor_count = len(spec.monitors)
             for name in ("indices", "weights", "freqs", "masks", "counts", "codes", "windows", "affine"):
                 setattr(s.dft, name, buf(getattr(a, name)))
+            K, P = (int(v) for v in a.indices.shape[2:])
+            self.slot_samples = (spec.ndim == 2 and schedule == "fused" and a.indices.numel() > 0
+                                 and slot_samples_fit(len(spec.monitors), K, P, self.dft_batch))
+            if self.slot_samples:
+                comps = [COMPONENT_INDEX[c] for c in self.active]
+                order, first = _dft_slots(a, comps, [self.shapes[c] for c in COMPONENTS], lattice)
+                s.dft.slot_order, s.dft.slot_first = buf(order), buf(first)
         # Time-domain field recorders.
         if len(spec.recorders) > abi.FDTD_MAX_RECORDERS:
             raise ValueError(f"at most {abi.FDTD_MAX_RECORDERS} field recorders")
@@ -734,6 +795,9 @@ class DeviceProgram:
                 d.indices[q], d.weights[q] = buf(pi), buf(pw)
                 if spec.ndim == 2:
                     d.box[q][:] = _unit_box(rec.indices[q], rec.weights[q], self.shapes[c][-1])
+                    if d.box[q][2] == 0 and pi.shape[0] == 1 and pi.numel() > 0:
+                        order, first = _recorder_slots(pi, pw, self.shapes[c], lattice)
+                        d.order[q], d.first[q] = buf(order.reshape(-1)), buf(first)
                 counts.append(int(pi.shape[1]))
             self.recorders.append(counts)
         self._times_for(max(int(spec.total_steps), 1))
@@ -879,10 +943,10 @@ class DeviceState:
         self.dft_w = torch.zeros(nw, dtype=torch.float32, device=dev)
         self.dft_samples = None
         if a is not None and program.dft_batch > 1:
-            # Per buffered step: the interpolated samples, or in 2D every
-            # gather slot's field value (FdtdDft.samples).
+            # Per buffered step: the interpolated samples, or every gather
+            # slot's field value (FdtdDft.samples).
             M, _six, K, P = (int(v) for v in a.indices.shape)
-            shape = (M, 6, K * P) if program.ndim == 2 else (M, 6, P)
+            shape = (M, 6, K * P) if program.slot_samples else (M, 6, P)
             self.dft_samples = torch.empty((program.dft_batch, *shape), dtype=torch.float32, device=dev)
         self.records = []
         for rec, counts in zip(program.spec.recorders, program.recorders):

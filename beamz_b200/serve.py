@@ -63,6 +63,8 @@ def estimate_bytes(spec: ProgramSpec, schedule: str = "fused") -> int:
     """Device bytes one simulation holds: two field banks (one for the phase
     schedule), CPML memories (H double-banked), material, DFT arena, field
     recorders, clock."""
+    from .runtime import slot_samples_fit
+
     active = active_components(spec.ndim, spec.polarization)
     shapes = {c: component_shape(c, spec.grid_shape, spec.polarization) for c in COMPONENTS}
     banks = 2 if schedule == "fused" else 1
@@ -78,10 +80,13 @@ def estimate_bytes(spec: ProgramSpec, schedule: str = "fused") -> int:
     e_banks = banks if spec.ndim == 2 else 1  # 2D programs double-bank the E memories too
     psi += sum(int(np.prod(t.psi_shape(shapes[t.component]))) * 4 * e_banks for t in spec.e_terms)
     dft = 0
-    for m in spec.monitors:
-        points = max(int(np.asarray(ix).shape[0]) for ix in m.indices)
-        slots = max(np.asarray(ix).size // max(1, len(ix)) for ix in m.indices)
-        per = slots if spec.ndim == 2 else 1  # sample batch: every slot's value in 2D
+    plans = [(max(int(np.asarray(ix).shape[0]) for ix in m.indices),
+              max(np.asarray(ix).size // max(1, len(ix)) for ix in m.indices)) for m in spec.monitors]
+    most = (max(p for p, _ in plans), max(k for _, k in plans)) if plans else (0, 1)
+    # The sample batch holds every slot's value in 2D, where that fits.
+    by_slot = spec.ndim == 2 and slot_samples_fit(len(plans), most[1], most[0])
+    for m, (points, slots) in zip(spec.monitors, plans):
+        per = slots if by_slot else 1
         dft += 6 * len(m.freqs) * points * 8 * 2 + 6 * points * 8 * 8 + 16 * 6 * points * 4 * per
     records = 0
     for r in spec.recorders:

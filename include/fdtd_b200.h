@@ -24,7 +24,7 @@ extern "C" {
 #endif
 
 /* Bumped whenever a struct below changes layout (beamz: abi_layout.json "abi_version"). */
-#define FDTD_ABI_VERSION 14
+#define FDTD_ABI_VERSION 15
 
 /* Element types (beamz: cuda/src/launch.h:6-10, plus U8 for voxel ids and F64
  * for reduction results). */
@@ -202,6 +202,16 @@ typedef struct FdtdDft {
    * packed plan only where the plan has exactly that form (plane monitors on
    * uniform coordinates do). */
   FdtdBuffer affine;
+  /* 2D programs, optional: which gather slots read which part of the grid.
+   * slot_order S32 [n <= M * 6 * K * P] lists offsets into `indices`, the
+   * slots that are sampled (active component, nonzero mask, nonzero weight up to
+   * the point's first zero one, cell on the grid) sorted by component, row and
+   * column of their cell; slot_first S32 [3, Y + 1, ceil((X + 1) / 16) + 1]: the
+   * number of them before 16-column block b of row j of the a-th active
+   * component.  fdtd_launch_program advances several steps per launch only with
+   * them: each tile reads its own slots. */
+  FdtdBuffer slot_order;
+  FdtdBuffer slot_first;
 } FdtdDft;
 
 /* A time-domain field recorder (beamz: FieldRecorder, compiled by
@@ -234,6 +244,12 @@ typedef struct FdtdRecorder {
    * unit weights in row order, as (y0, x0, ny, nx); ny = 0: it is not.  The
    * indices and weights still describe it. */
   int32_t box[6][4];
+  /* 2D programs, optional: FdtdDft.slot_order / slot_first of value set q's plan
+   * (order S32 [V], the values with a zero weight or no cell last; first S32
+   * [Y + 1, ceil((X + 1) / 16) + 1]).  Sets that are neither whole components nor
+   * boxes need them to advance several steps per launch. */
+  FdtdBuffer order[6];
+  FdtdBuffer first[6];
 } FdtdRecorder;
 
 /* A complete step program (replaces BeamzLaunch + BeamzProgramLaunch,
