@@ -461,8 +461,10 @@ __global__ void __launch_bounds__(kAdjThreads) adj_curl_kernel(Step3D p, AdjDev 
   const int bz = a.box_hi[0] - a.box_lo[0], by = a.box_hi[1] - a.box_lo[1], bx = a.box_hi[2] - a.box_lo[2];
   const int64_t n = static_cast<int64_t>(bz) * by * bx;
   const float res = p.res;
-  const Dims dx = component_dims(3, p.Z, p.Y, p.X), dy = component_dims(4, p.Z, p.Y, p.X),
-             dz = component_dims(5, p.Z, p.Y, p.X);
+  const Dims lattice = {p.Z + 1, p.Y + 1, p.pitch};  // per-site programs on the pitched layout
+  const Dims dx = p.site ? lattice : component_dims(3, p.Z, p.Y, p.X);
+  const Dims dy = p.site ? lattice : component_dims(4, p.Z, p.Y, p.X);
+  const Dims dz = p.site ? lattice : component_dims(5, p.Z, p.Y, p.X);
   for (int64_t b = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; b < n;
        b += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int i = a.box_lo[2] + static_cast<int>(b % bx);

@@ -331,6 +331,16 @@ SlotOrder slot_order(const FdtdBuffer& order, const FdtdBuffer& first) {
   return s;
 }
 
+// A program as the phase-level entries take it: one bank, dense -- or, of the
+// fused programs, a lossless per-site one on the pitched layout, whose current
+// bank is stepped in place.
+int validate_phase(const FdtdProgram& program, FdtdProgram* p) {
+  *p = program;
+  const bool pitched_site = p->layout == FDTD_LAYOUT_PITCHED && p->material_kind == FDTD_MATERIAL_SITE;
+  if (!pitched_site) p->schedule = FDTD_SCHEDULE_PHASES;
+  return validate(*p);
+}
+
 // Device view of recorder r reading the component arrays of `bank`.
 RecorderDev recorder_dev(const FdtdProgram& p, const Layout& L, int r, const FdtdBuffer* bank) {
   const FdtdRecorder& rec = p.recorders[r];
@@ -891,10 +901,8 @@ int fdtd_validate(const FdtdProgram* program) {
 
 int fdtd_launch_phase(void* stream, const FdtdProgram* program, int32_t phase) {
   if (program == nullptr || (phase != 0 && phase != 1)) return fdtd::kInvalid;
-  if (program->layout != FDTD_LAYOUT_DENSE) return fdtd::kInvalid;
-  FdtdProgram p = *program;
-  p.schedule = FDTD_SCHEDULE_PHASES;
-  const int v = fdtd::validate(p);
+  FdtdProgram p;
+  const int v = fdtd::validate_phase(*program, &p);
   if (v != 0) return v;
   fdtd::Layout L;
   fdtd::layout_of(p, &L);
@@ -915,9 +923,8 @@ int fdtd_launch_program(void* stream, const FdtdProgram* program) {
 
 int fdtd_apply_sources(void* stream, const FdtdProgram* program, int32_t timing, int32_t step_offset) {
   if (program == nullptr) return fdtd::kInvalid;
-  FdtdProgram p = *program;
-  p.schedule = FDTD_SCHEDULE_PHASES;
-  const int v = fdtd::validate(p);
+  FdtdProgram p;
+  const int v = fdtd::validate_phase(*program, &p);
   if (v != 0) return v;
   if (timing < FDTD_TIMING_PRE_E || timing > FDTD_TIMING_E) return fdtd::kInvalid;
   fdtd::Layout L;
@@ -928,9 +935,8 @@ int fdtd_apply_sources(void* stream, const FdtdProgram* program, int32_t timing,
 
 int fdtd_accumulate_dft(void* stream, const FdtdProgram* program, int32_t step_offset) {
   if (program == nullptr) return fdtd::kInvalid;
-  FdtdProgram p = *program;
-  p.schedule = FDTD_SCHEDULE_PHASES;
-  const int v = fdtd::validate(p);
+  FdtdProgram p;
+  const int v = fdtd::validate_phase(*program, &p);
   if (v != 0) return v;
   if (p.dft.monitor_count == 0) return 0;
   return static_cast<int>(fdtd::launch_dft(static_cast<cudaStream_t>(stream), fdtd::make_dft(p, p.fields),
@@ -939,9 +945,8 @@ int fdtd_accumulate_dft(void* stream, const FdtdProgram* program, int32_t step_o
 
 int fdtd_record_fields(void* stream, const FdtdProgram* program, int32_t step_offset) {
   if (program == nullptr) return fdtd::kInvalid;
-  FdtdProgram p = *program;
-  p.schedule = FDTD_SCHEDULE_PHASES;
-  const int v = fdtd::validate(p);
+  FdtdProgram p;
+  const int v = fdtd::validate_phase(*program, &p);
   if (v != 0) return v;
   fdtd::Layout L;
   fdtd::layout_of(p, &L);
@@ -972,11 +977,11 @@ namespace {
 
 bool f32_sized(const FdtdBuffer& b, int64_t n) { return is_f32(b) && b.data != nullptr && elements(b) == n; }
 
-// Shared checks of an adjoint call: a valid dense phase program and a box
-// whose curl needs no ghost, wall or CPML handling.
+// Shared checks of an adjoint call on a valid phase program (dense, but for the
+// curl alone): a box whose curl needs no ghost, wall or CPML handling.
 int check_adjoint(const FdtdProgram& p, const FdtdAdjointStep& a, const Layout& L, bool need_box, int64_t steps = 1) {
   if (a.abi_version != FDTD_ABI_VERSION) return kInvalid;
-  if (p.layout != FDTD_LAYOUT_DENSE) return kInvalid;
+  if (p.layout != FDTD_LAYOUT_DENSE && !need_box) return kInvalid;
   const int64_t bz = a.box_hi[0] - a.box_lo[0], by = a.box_hi[1] - a.box_lo[1], bx = a.box_hi[2] - a.box_lo[2];
   bool any_box = false;
   for (int c = 0; c < 3; ++c) any_box = any_box || a.curl[c].data != nullptr || a.grad[c].data != nullptr;
@@ -1113,9 +1118,8 @@ int fdtd_adjoint_steps(void* stream, const FdtdProgram* adjoint, const FdtdAdjoi
 
 int fdtd_adjoint_curl(void* stream, const FdtdProgram* forward, const FdtdAdjointStep* a) {
   if (forward == nullptr || a == nullptr) return fdtd::kInvalid;
-  FdtdProgram p = *forward;
-  p.schedule = FDTD_SCHEDULE_PHASES;
-  const int v = fdtd::validate(p);
+  FdtdProgram p;
+  const int v = fdtd::validate_phase(*forward, &p);
   if (v != 0) return v;
   fdtd::Layout L;
   fdtd::layout_of(p, &L);

@@ -85,7 +85,8 @@ enum {
  *          FDTD_MATERIAL_CODEBOOK, or with FDTD_MATERIAL_SITE for lossless
  *          materials: e_source[c] then holds E <- E + source * curl's source on
  *          the fields' (Z+1, Y+1, pitch) shape (e_decay is not read; isotropic
- *          grids, exact arithmetic).  fdtd_copy_component converts between
+ *          grids, exact arithmetic).  The phase-level entries take the latter
+ *          too, not the codebook.  fdtd_copy_component converts between
  *          layouts. */
 enum {
   FDTD_LAYOUT_DENSE = 0,
@@ -348,7 +349,10 @@ int fdtd_validate(const FdtdProgram* program);
 
 /* One in-place half step: phase 0 = H from E, phase 1 = E from H, including
  * CPML psi and PEC zeroing of constrained cells (beamz: BeamzLaunchStreamed,
- * cuda/src/update.cu:919-971; beamz/simulation/cuda/runtime.py:184/234). */
+ * cuda/src/update.cu:919-971; beamz/simulation/cuda/runtime.py:184/234).  This
+ * and the other phase-level entries (sources, DFT, records, the design-box curl)
+ * act on `fields` and `psi` of dense programs and of FDTD_MATERIAL_SITE programs
+ * on the pitched layout. */
 int fdtd_launch_phase(void* stream, const FdtdProgram* program, int32_t phase);
 
 /* Enqueue program->nsteps complete leapfrog steps -- sources at their three
