@@ -88,13 +88,14 @@ class AdjointProblem:
     def _forward_layout(self, spec: ProgramSpec) -> str:
         """3D forward runs take the class step's layout with per-site
         coefficients (the step is bit-identical and four times as fast as the
-        dense one); metric grids, lossy materials and checkpointed runs, whose
-        curls are read from dense H, stay on the dense layout."""
-        from .runtime import lossless_site_sources
+        dense one); metric grids, lossy materials, checkpointed runs, whose
+        curls are read from dense H, and grids whose padded fields would reach
+        2^31 elements stay on the dense layout."""
+        from .runtime import lossless_site_sources, pitched_size_ok
 
         uniform = all(np.ndim(v) == 0 for pair in spec.h_coefficients().values() for v in pair)
         if (spec.ndim != 3 or spec.metrics is not None or self.curl_record is None or not uniform
-                or lossless_site_sources(spec) is None):
+                or lossless_site_sources(spec) is None or not pitched_size_ok(spec.grid_shape)):
             return "dense"
         return "site"
 

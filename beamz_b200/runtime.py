@@ -493,6 +493,13 @@ def _unit_box(indices, weights, row: int):
     return (y0, x0, ny, nx) if np.array_equal(box.reshape(-1), i) else (0, 0, 0, 0)
 
 
+def pitched_size_ok(grid_shape) -> bool:
+    """Does a field on the pitched layout stay below 2^31 elements (FdtdProgram's
+    limit)?  Its padding can pass it where the dense components do not."""
+    nz, ny, nx = (int(v) for v in grid_shape)
+    return (nz + 1) * (ny + 1) * (-(-(nx + 1) // 4) * 4) < 2**31
+
+
 class DeviceProgram:
     """A compiled program: every static input of the step, resident on the device."""
 
@@ -529,10 +536,10 @@ class DeviceProgram:
         # component (lossless per-site material on an isotropic grid); "auto"
         # takes it where the codebook does not hold the material's values.
         site_ok = (site_sources is not None and schedule == "fused" and h_uniform and spec.metrics is None
-                   and arithmetic == "exact" and step_kernel == "classes")
+                   and arithmetic == "exact" and step_kernel == "classes" and pitched_size_ok(spec.grid_shape))
         if layout == "site" and not site_ok:
             raise ValueError("the site layout needs a lossless per-site 3D program on an isotropic grid, the fused "
-                             "schedule and exact arithmetic")
+                             "schedule and exact arithmetic, and fewer than 2^31 elements per padded field")
         self.per_site = layout == "site"
         if self.per_site:
             layout = "pitched"
