@@ -345,7 +345,8 @@ __global__ void __launch_bounds__(kAdjX* kAdjY, 8) adj_e_pass(const __grid_const
 template <int Active>
 __global__ void __launch_bounds__(kAdjThreads) adj_h_finish(const __grid_constant__ Step3D p,
                                                             const __grid_constant__ AdjDev a) {
-  const int first = blockIdx.x * kAdjThreads + threadIdx.x, stride = gridDim.x * kAdjThreads;
+  // Unsigned: a component may hold 2^31 - 1 elements, and the last stride passes that.
+  const unsigned first = blockIdx.x * kAdjThreads + threadIdx.x, stride = gridDim.x * kAdjThreads;
 #pragma unroll
   for (int hc = 0; hc < 3; ++hc) {
     if (!((Active >> (3 + hc)) & 1) || static_cast<int>(blockIdx.y) != hc) continue;
@@ -365,8 +366,8 @@ __global__ void __launch_bounds__(kAdjThreads) adj_h_finish(const __grid_constan
         const int w = term.low + term.high;
         if (w == 0) continue;
         const Dims sd = {axis == 0 ? w : d.z, axis == 1 ? w : d.y, axis == 2 ? w : d.x};  // the slab
-        const int n = sd.z * sd.y * sd.x;
-        for (int e = first; e < n; e += stride) {
+        const unsigned n = sd.z * sd.y * sd.x;
+        for (unsigned e = first; e < n; e += stride) {
           const int r = e / sd.x;
           int i = e - r * sd.x, k = r / sd.y, j = r - k * sd.y;
           int& x = axis == 0 ? k : (axis == 1 ? j : i);
@@ -376,8 +377,8 @@ __global__ void __launch_bounds__(kAdjThreads) adj_h_finish(const __grid_constan
       }
       continue;
     }
-    const int n = d.z * d.y * d.x;
-    for (int e = first; e < n; e += stride) {
+    const unsigned n = d.z * d.y * d.x;
+    for (unsigned e = first; e < n; e += stride) {
       const int r = e / d.x;
       const int i = e - r * d.x, k = r / d.y, j = r - k * d.y;
       const float mu = a.lam[3 + hc][e];
