@@ -1113,6 +1113,7 @@ int fdtd_adjoint_step_noalloc(void* stream, const FdtdProgram* adjoint, const Fd
 }
 
 int fdtd_adjoint_steps(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a, int32_t count) {
+  if (a != nullptr && a->step < count - 1) return fdtd::kInvalid;  // a run ends at step 0
   return fdtd::run_adjoint(stream, adjoint, a, 2, count);
 }
 

@@ -441,7 +441,8 @@ int fdtd_adjoint_step_noalloc(void* stream, const FdtdProgram* adjoint, const Fd
 /* `count` adjoint steps in a row, a->step first, then each earlier one, enqueued
  * by one call.  As fdtd_adjoint_step, without scratch, and with a->curl[c]
  * holding the curls of steps a->step - count + 1 .. a->step in ascending order
- * (F32 [count, box]). */
+ * (F32 [count, box]).  A run that would pass step 0 (count > a->step + 1) is
+ * rejected before any work is enqueued. */
 int fdtd_adjoint_steps(void* stream, const FdtdProgram* adjoint, const FdtdAdjointStep* a, int32_t count);
 
 /* Write the forward curl of each active E component over `a`'s box into
