@@ -167,7 +167,7 @@ __device__ __forceinline__ void own_slots(const Block2D& q, const SlotOrder& so,
   const int j = t.j + row;
   if (j >= d.y) return;
   const int blocks = (q.p.X + kSlotBlock) / kSlotBlock;
-  const int* first = so.first + (a * (q.p.Y + 1) + j) * (blocks + 1);
+  const int* first = so.first + (a * (q.p.Y + 1) + j) * blocks;
   const int lo = max(__ldg(first + t.i / kSlotBlock), 0);
   const int hi = min(__ldg(first + min((t.i + g.TX + kSlotBlock - 1) / kSlotBlock, blocks)), so.n);
   const int from = j * d.x + t.i, width = min(g.TX, d.x - t.i);  // the row's own cells
@@ -209,7 +209,7 @@ __device__ __forceinline__ void own_values(const Block2D& q, int only, const Til
                        [&](int at, int cell) { emit(cell, at, rec.w[v][at], n * 8 + v); });
       if (t.n != 0) continue;
       const int blocks = (q.p.X + kSlotBlock) / kSlotBlock;
-      for (int e = max(so.first[(q.p.Y + 1) * (blocks + 1) - 1], 0) + tid; e < V; e += nthreads) {
+      for (int e = max(so.first[(q.p.Y + 1) * blocks], 0) + tid; e < V; e += nthreads) {
         const int at = so.order[e];
         if (at >= 0 && at < V) emit(-1, at, 0.0f, n * 8 + v);
       }

@@ -96,7 +96,7 @@ bool slot_order_ok(const FdtdProgram& p, const Layout& L, const FdtdBuffer& orde
   if (p.ndim != 2 || order.data == nullptr || first.data == nullptr) return false;
   const int64_t blocks = (L.X + kSlotBlock) / kSlotBlock;  // of X + 1 columns
   return order.element_type == FDTD_S32 && first.element_type == FDTD_S32 && elements(order) >= 0 &&
-         elements(order) <= most && elements(first) == comps * (L.Y + 1) * (blocks + 1);
+         elements(order) <= most && elements(first) == comps * (L.Y + 1) * blocks + 1;
 }
 
 int validate(const FdtdProgram& p) {

@@ -405,22 +405,47 @@ def _affine_plan(idx, w):
             + [int(v) for v in bits] + [0] * (8 - k))
 
 
-def _slots_by_cell(cells, live, widths, rows: int, cols: int):
+def _slots_by_cell(cells, live, groups, lattice):
     """Gather slots sorted by the cell they read (FdtdDft.slot_order): positions
-    in the flattened ``cells`` [components, n], live ones first by component, row
-    and column, and per component, row and 16-column block of a rows x cols
-    lattice the number of slots before it.  ``widths``: row length of each
-    component."""
+    in the flattened ``cells``, live ones first by component, row and column, and
+    the number of them before each 16-column block of each row of each component.
+    ``groups``: the components' row lengths and sizes, along cells' dimension 1."""
     torch = _torch()
-    dev = cells.device
-    blocks = -(-cols // 16)
-    group = torch.arange(cells.shape[0] * rows, device=dev).view(-1, rows, 1)
-    width = torch.tensor(widths, device=dev).view(-1, 1)
-    key = (torch.div(cells, width, rounding_mode="floor") + group[:, 0]) * (16 * blocks) + cells % width
-    key = torch.where(live, key, group.numel() * 16 * blocks).reshape(-1)
-    key, order = torch.sort(key)
-    first = torch.searchsorted(key, group * (16 * blocks) + 16 * torch.arange(blocks + 1, device=dev))
-    return order, first.to(torch.int32)
+    rows, cols = lattice
+    row_keys = 16 * -(-cols // 16)
+    n = len(groups)
+    width, size, base = torch.tensor([[w for w, _ in groups], [z for _, z in groups],
+                                      [a * rows * row_keys for a in range(n)]], device=cells.device).view(3, n, 1, 1)
+    live = live & (cells >= 0) & (cells < size)
+    key = cells + torch.div(cells, width, rounding_mode="floor") * (row_keys - width) + base
+    key, order = torch.sort(torch.where(live, key, n * rows * row_keys).reshape(-1))
+    blocks = torch.arange(0, n * rows * row_keys + 1, 16, device=cells.device)
+    return order, torch.searchsorted(key, blocks, out_int32=True)
+
+
+def _dft_slots(arena, components, shapes, lattice):
+    """FdtdDft.slot_order and slot_first of a 2D program's packed plan."""
+    torch = _torch()
+    lo, hi = components[0], components[-1] + 1
+
+    def pick(t):  # the active components' parts of a [M, 6, ...] array
+        return t[:, lo:hi] if hi - lo == len(components) else torch.cat([t[:, c:c + 1] for c in components], dim=1)
+
+    live = pick(arena.weights) != 0
+    if live.shape[2] > 1:
+        live = live.cumprod(dim=2).bool()  # a zero weight ends a point's gather
+    live = live & (pick(arena.masks) != 0)[:, :, None, None]
+    order, first = _slots_by_cell(pick(arena.indices), live,
+                                  [(int(shapes[c][1]), int(np.prod(shapes[c]))) for c in components], lattice)
+    at = torch.arange(arena.indices.numel(), dtype=torch.int32, device=first.device).view(arena.indices.shape)
+    return pick(at).reshape(-1)[order], first
+
+
+def _recorder_slots(indices, weights, shape, lattice):
+    """FdtdRecorder.order and first of one packed one-slot plan of a 2D program."""
+    order, first = _slots_by_cell(indices[:, None, None], (weights != 0)[:, None, None],
+                                  [(int(shape[1]), int(np.prod(shape)))], lattice)
+    return order.to(indices.dtype), first
 
 
 def slot_samples_fit(monitors: int, slots: int, points: int, batch: int = 16) -> bool:
@@ -431,30 +456,6 @@ def slot_samples_fit(monitors: int, slots: int, points: int, batch: int = 16) ->
     10.8 us per step against 19 in single steps at 200 x 200 (61 MB), but 25.3
     against 23.9 at 400 x 400 (245 MB)."""
     return batch >= 2 and 4 * batch * monitors * 6 * slots * points <= (1 << 30 if slots == 1 else 1 << 27)
-
-
-def _dft_slots(arena, components, shapes, lattice):
-    """FdtdDft.slot_order and slot_first of a 2D program's packed plan."""
-    torch = _torch()
-    M, _six, K, P = (int(v) for v in arena.indices.shape)
-    n = len(components)
-    at = torch.arange(arena.indices.numel(), device=arena.indices.device).view(M, 6, K, P)[:, components]
-    cells = arena.indices[:, components].long()
-    size = torch.tensor([int(np.prod(shapes[c])) for c in components], device=cells.device).view(1, n, 1, 1)
-    live = (arena.weights[:, components] != 0).cumprod(dim=2).bool()  # a zero weight ends a point's gather
-    live &= (cells >= 0) & (cells < size) & (arena.masks[:, components] != 0).view(M, n, 1, 1)
-    live &= torch.arange(P, device=cells.device) < arena.counts[:, 1].view(M, 1, 1, 1)
-    flat = lambda t: t.transpose(0, 1).reshape(n, -1)  # noqa: E731
-    order, first = _slots_by_cell(flat(cells), flat(live), [int(shapes[c][1]) for c in components], *lattice)
-    return flat(at).reshape(-1)[order].to(torch.int32), first
-
-
-def _recorder_slots(indices, weights, shape, lattice):
-    """FdtdRecorder.order and first of one packed one-slot plan of a 2D program."""
-    cells = indices.long()
-    live = (weights != 0) & (cells >= 0) & (cells < int(np.prod(shape)))
-    order, first = _slots_by_cell(cells, live, [int(shape[1])], *lattice)
-    return order.to(indices.dtype), first
 
 
 def _pack_plan(lib, stream, indices, weights, dims, strides, device):
@@ -804,7 +805,7 @@ class DeviceProgram:
                     d.box[q][:] = _unit_box(rec.indices[q], rec.weights[q], self.shapes[c][-1])
                     if d.box[q][2] == 0 and pi.shape[0] == 1 and pi.numel() > 0:
                         order, first = _recorder_slots(pi, pw, self.shapes[c], lattice)
-                        d.order[q], d.first[q] = buf(order.reshape(-1)), buf(first)
+                        d.order[q], d.first[q] = buf(order), buf(first)
                 counts.append(int(pi.shape[1]))
             self.recorders.append(counts)
         self._times_for(max(int(spec.total_steps), 1))

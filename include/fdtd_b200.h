@@ -207,10 +207,11 @@ typedef struct FdtdDft {
    * slot_order S32 [n <= M * 6 * K * P] lists offsets into `indices`, the
    * slots that are sampled (active component, nonzero mask, nonzero weight up to
    * the point's first zero one, cell on the grid) sorted by component, row and
-   * column of their cell; slot_first S32 [3, Y + 1, ceil((X + 1) / 16) + 1]: the
-   * number of them before 16-column block b of row j of the a-th active
-   * component.  fdtd_launch_program advances several steps per launch only with
-   * them: each tile reads its own slots. */
+   * column of their cell; slot_first S32 [3 (Y + 1) B + 1], B = ceil((X + 1) / 16):
+   * element (a (Y + 1) + j) B + b the number of them before 16-column block b of
+   * row j of the a-th active component, the last one their number.
+   * fdtd_launch_program advances several steps per launch only with them: each
+   * tile reads its own slots. */
   FdtdBuffer slot_order;
   FdtdBuffer slot_first;
 } FdtdDft;
@@ -247,7 +248,7 @@ typedef struct FdtdRecorder {
   int32_t box[6][4];
   /* 2D programs, optional: FdtdDft.slot_order / slot_first of value set q's plan
    * (order S32 [V], the values with a zero weight or no cell last; first S32
-   * [Y + 1, ceil((X + 1) / 16) + 1]).  Sets that are neither whole components nor
+   * [(Y + 1) B + 1]).  Sets that are neither whole components nor
    * boxes need them to advance several steps per launch. */
   FdtdBuffer order[6];
   FdtdBuffer first[6];

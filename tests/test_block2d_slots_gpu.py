@@ -127,7 +127,7 @@ def test_slot_tables_of_other_sizes_are_rejected():
 
     s = prog.fill(st, 1)
     assert prog.lib.fdtd_validate(ctypes.byref(s)) == 0
-    s.dft.slot_first.dims[1] -= 1
+    s.dft.slot_first.dims[0] -= 1
     assert prog.lib.fdtd_validate(ctypes.byref(s)) == 1
     s = prog.fill(st, 1)
     s.dft.slot_order.data = None
