@@ -52,6 +52,7 @@ EXPORTED_SYMBOLS = (
     "fdtd_field_diagnostics",
     "fdtd_dft_change",
     "fdtd_pack_gather",
+    "fdtd_slot_order",
     "fdtd_voxel_histogram",
     "fdtd_monitor_reduce",
     "fdtd_adjoint_step_noalloc",
@@ -170,6 +171,22 @@ class FdtdGatherPack(ctypes.Structure):
         ("dims", ctypes.c_int32 * 3),
         ("row", ctypes.c_int64),
         ("plane", ctypes.c_int64),
+    ]
+
+
+class FdtdSlotOrder(ctypes.Structure):
+    _fields_ = [
+        ("indices", FdtdBuffer),
+        ("weights", FdtdBuffer),
+        ("masks", FdtdBuffer),
+        ("component_count", ctypes.c_int32),
+        ("components", ctypes.c_int32 * 3),
+        ("widths", ctypes.c_int32 * 3),
+        ("heights", ctypes.c_int32 * 3),
+        ("rows", ctypes.c_int32),
+        ("cols", ctypes.c_int32),
+        ("order", FdtdBuffer),
+        ("first", FdtdBuffer),
     ]
 
 
@@ -354,6 +371,8 @@ def load_library(path: str | None = None):
         lib.fdtd_dft_change.restype = ctypes.c_int
         lib.fdtd_pack_gather.argtypes = [ctypes.c_void_p, ctypes.POINTER(FdtdGatherPack)]
         lib.fdtd_pack_gather.restype = ctypes.c_int
+        lib.fdtd_slot_order.argtypes = [ctypes.c_void_p, ctypes.POINTER(FdtdSlotOrder)]
+        lib.fdtd_slot_order.restype = ctypes.c_int
         lib.fdtd_voxel_histogram.argtypes = [ctypes.c_void_p, ctypes.POINTER(FdtdBuffer), ctypes.POINTER(FdtdBuffer)]
         lib.fdtd_voxel_histogram.restype = ctypes.c_int
         lib.fdtd_monitor_reduce.argtypes = [ctypes.c_void_p, ctypes.POINTER(FdtdProgram),

@@ -267,6 +267,21 @@ struct GatherPackDev {
 };
 
 cudaError_t launch_gather_pack(cudaStream_t s, const GatherPackDev& g);
+
+// The slots of packed plans sorted by cell (planner.cu; see FdtdSlotOrder).
+struct SlotSortDev {
+  const int* idx = nullptr;     // [M, C, K, P]
+  const float* w = nullptr;
+  const float* masks = nullptr; // [M, C] or null
+  int M = 0, C = 0, K = 0, P = 0;
+  int n = 0;                    // components sorted, of the C
+  int comp[3] = {0, 0, 0};
+  int width[3] = {0, 0, 0}, height[3] = {0, 0, 0};
+  int rows = 0, blocks = 0;     // lattice rows, 16-column blocks per row
+  int* order = nullptr;         // [M * n * K * P]
+  int* first = nullptr;         // [n * rows * blocks + 1]
+};
+cudaError_t launch_slot_order(cudaStream_t s, const SlotSortDev& d);
 cudaError_t launch_voxel_histogram(cudaStream_t s, const uint8_t* v, int64_t n, int* counts);
 
 // Field diagnostics (diag.cu): one component's view.

@@ -1268,6 +1268,47 @@ int fdtd_pack_gather(void* stream, const FdtdGatherPack* g) {
   return static_cast<int>(fdtd::launch_gather_pack(static_cast<cudaStream_t>(stream), d));
 }
 
+int fdtd_slot_order(void* stream, const FdtdSlotOrder* g) {
+  if (g == nullptr) return fdtd::kInvalid;
+  const FdtdBuffer &ix = g->indices, &w = g->weights, &mk = g->masks, &order = g->order, &first = g->first;
+  if (ix.element_type != FDTD_S32 || !fdtd::is_f32(w) || order.element_type != FDTD_S32 ||
+      first.element_type != FDTD_S32 || ix.rank != 4 || w.rank != 4)
+    return fdtd::kInvalid;
+  for (int a = 0; a < 4; ++a)
+    if (ix.dims[a] != w.dims[a] || ix.dims[a] < 1) return fdtd::kInvalid;
+  const int64_t M = ix.dims[0], C = ix.dims[1];
+  if (fdtd::elements(ix) >= (int64_t{1} << 31) || g->component_count < 1 || g->component_count > 3) return fdtd::kInvalid;
+  if (g->rows < 1 || g->cols < 1) return fdtd::kInvalid;
+  fdtd::SlotSortDev d;
+  d.M = static_cast<int>(M);
+  d.C = static_cast<int>(C);
+  d.K = static_cast<int>(ix.dims[2]);
+  d.P = static_cast<int>(ix.dims[3]);
+  d.n = g->component_count;
+  for (int a = 0; a < d.n; ++a) {
+    if (g->components[a] < 0 || g->components[a] >= C || g->widths[a] < 1 || g->widths[a] > g->cols ||
+        g->heights[a] < 1 || g->heights[a] > g->rows)
+      return fdtd::kInvalid;
+    d.comp[a] = g->components[a];
+    d.width[a] = g->widths[a];
+    d.height[a] = g->heights[a];
+  }
+  d.rows = g->rows;
+  d.blocks = (g->cols + fdtd::kSlotBlock - 1) / fdtd::kSlotBlock;
+  const int64_t bins = static_cast<int64_t>(d.n) * d.rows * d.blocks + 1;
+  if (bins >= (int64_t{1} << 31) || fdtd::elements(first) != bins ||
+      fdtd::elements(order) != M * d.n * ix.dims[2] * ix.dims[3])
+    return fdtd::kInvalid;
+  if (mk.data != nullptr && (!fdtd::is_f32(mk) || fdtd::elements(mk) != M * C)) return fdtd::kInvalid;
+  if (ix.data == nullptr || w.data == nullptr || order.data == nullptr || first.data == nullptr) return fdtd::kInvalid;
+  d.idx = static_cast<const int*>(ix.data);
+  d.w = static_cast<const float*>(w.data);
+  d.masks = static_cast<const float*>(mk.data);
+  d.order = static_cast<int*>(order.data);
+  d.first = static_cast<int*>(first.data);
+  return static_cast<int>(fdtd::launch_slot_order(static_cast<cudaStream_t>(stream), d));
+}
+
 int fdtd_voxel_histogram(void* stream, const FdtdBuffer* voxels, const FdtdBuffer* counts) {
   if (voxels == nullptr || counts == nullptr) return fdtd::kInvalid;
   if (voxels->element_type != FDTD_U8 || counts->element_type != FDTD_S32 || fdtd::elements(*counts) != 256 ||

@@ -405,47 +405,24 @@ def _affine_plan(idx, w):
             + [int(v) for v in bits] + [0] * (8 - k))
 
 
-def _slots_by_cell(cells, live, groups, lattice):
-    """Gather slots sorted by the cell they read (FdtdDft.slot_order): positions
-    in the flattened ``cells``, live ones first by component, row and column, and
-    the number of them before each 16-column block of each row of each component.
-    ``groups``: the components' row lengths and sizes, along cells' dimension 1."""
+def _slots_by_cell(lib, stream, indices, weights, masks, components, shapes, lattice):
+    """The slots of a packed [M, C, K, P] plan sorted by the cell that they read
+    (fdtd_slot_order): order and first of the chosen components, with stored
+    ``shapes``, on a (Y + 1, X + 1) ``lattice``."""
     torch = _torch()
-    rows, cols = lattice
-    row_keys = 16 * -(-cols // 16)
-    n = len(groups)
-    width, size, base = torch.tensor([[w for w, _ in groups], [z for _, z in groups],
-                                      [a * rows * row_keys for a in range(n)]], device=cells.device).view(3, n, 1, 1)
-    live = live & (cells >= 0) & (cells < size)
-    key = cells + torch.div(cells, width, rounding_mode="floor") * (row_keys - width) + base
-    key, order = torch.sort(torch.where(live, key, n * rows * row_keys).reshape(-1))
-    blocks = torch.arange(0, n * rows * row_keys + 1, 16, device=cells.device)
-    return order, torch.searchsorted(key, blocks, out_int32=True)
-
-
-def _dft_slots(arena, components, shapes, lattice):
-    """FdtdDft.slot_order and slot_first of a 2D program's packed plan."""
-    torch = _torch()
-    lo, hi = components[0], components[-1] + 1
-
-    def pick(t):  # the active components' parts of a [M, 6, ...] array
-        return t[:, lo:hi] if hi - lo == len(components) else torch.cat([t[:, c:c + 1] for c in components], dim=1)
-
-    live = pick(arena.weights) != 0
-    if live.shape[2] > 1:
-        live = live.cumprod(dim=2).bool()  # a zero weight ends a point's gather
-    live = live & (pick(arena.masks) != 0)[:, :, None, None]
-    order, first = _slots_by_cell(pick(arena.indices), live,
-                                  [(int(shapes[c][1]), int(np.prod(shapes[c]))) for c in components], lattice)
-    at = torch.arange(arena.indices.numel(), dtype=torch.int32, device=first.device).view(arena.indices.shape)
-    return pick(at).reshape(-1)[order], first
-
-
-def _recorder_slots(indices, weights, shape, lattice):
-    """FdtdRecorder.order and first of one packed one-slot plan of a 2D program."""
-    order, first = _slots_by_cell(indices[:, None, None], (weights != 0)[:, None, None],
-                                  [(int(shape[1]), int(np.prod(shape)))], lattice)
-    return order.to(indices.dtype), first
+    M, _c, K, P = (int(v) for v in indices.shape)
+    n, (rows, cols) = len(components), lattice
+    g = abi.FdtdSlotOrder()
+    g.component_count, g.rows, g.cols = n, rows, cols
+    for a, (c, shape) in enumerate(zip(components, shapes)):
+        g.components[a], g.heights[a], g.widths[a] = c, int(shape[0]), int(shape[1])
+    order = torch.empty(M * n * K * P, dtype=torch.int32, device=indices.device)
+    first = torch.empty(n * rows * -(-cols // 16) + 1, dtype=torch.int32, device=indices.device)
+    g.indices, g.weights, g.masks = abi.buffer_of(indices), abi.buffer_of(weights), abi.buffer_of(masks)
+    g.order, g.first = abi.buffer_of(order), abi.buffer_of(first)
+    abi.check(lib.fdtd_slot_order(stream, ctypes.byref(g)), "fdtd_slot_order")
+    torch.cuda.current_stream(indices.device).synchronize()  # before any stream of the program reads them
+    return order, first
 
 
 def slot_samples_fit(monitors: int, slots: int, points: int, batch: int = 16) -> bool:
@@ -761,6 +738,7 @@ class DeviceProgram:
                 s.metric_h[a] = buf(_f32(spec.metrics.along(f"e_to_h_{name}", n), dev))
                 s.metric_e[a] = buf(_f32(spec.metrics.along(f"h_to_e_{name}", n + 1), dev))
         # Monitors.
+        stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         lattice = tuple(int(v) + 1 for v in spec.grid_shape)
         self.arena = pack_dft_monitors(spec.monitors, dev, [self.shapes[c] for c in COMPONENTS], self._strides)
         self.slot_samples = False  # are every gather slot's values buffered (2D, several steps per launch)?
@@ -774,13 +752,13 @@ class DeviceProgram:
                                  and slot_samples_fit(len(spec.monitors), K, P, self.dft_batch))
             if self.slot_samples:
                 comps = [COMPONENT_INDEX[c] for c in self.active]
-                order, first = _dft_slots(a, comps, [self.shapes[c] for c in COMPONENTS], lattice)
+                order, first = _slots_by_cell(self.lib, stream, a.indices, a.weights, a.masks, comps,
+                                              [self.shapes[c] for c in self.active], lattice)
                 s.dft.slot_order, s.dft.slot_first = buf(order), buf(first)
         # Time-domain field recorders.
         if len(spec.recorders) > abi.FDTD_MAX_RECORDERS:
             raise ValueError(f"at most {abi.FDTD_MAX_RECORDERS} field recorders")
         self.recorders = []  # per recorder: values per record of each component
-        stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         s.recorder_count = len(spec.recorders)
         for r, rec in enumerate(spec.recorders):
             d = s.recorders[r]
@@ -804,7 +782,8 @@ class DeviceProgram:
                 if spec.ndim == 2:
                     d.box[q][:] = _unit_box(rec.indices[q], rec.weights[q], self.shapes[c][-1])
                     if d.box[q][2] == 0 and pi.shape[0] == 1 and pi.numel() > 0:
-                        order, first = _recorder_slots(pi, pw, self.shapes[c], lattice)
+                        order, first = _slots_by_cell(self.lib, stream, pi[None, None], pw[None, None], None, [0],
+                                                      [self.shapes[c]], lattice)
                         d.order[q], d.first[q] = buf(order), buf(first)
                 counts.append(int(pi.shape[1]))
             self.recorders.append(counts)

@@ -203,11 +203,11 @@ typedef struct FdtdDft {
    * packed plan only where the plan has exactly that form (plane monitors on
    * uniform coordinates do). */
   FdtdBuffer affine;
-  /* 2D programs, optional: which gather slots read which part of the grid.
-   * slot_order S32 [n <= M * 6 * K * P] lists offsets into `indices`, the
-   * slots that are sampled (active component, nonzero mask, nonzero weight up to
-   * the point's first zero one, cell on the grid) sorted by component, row and
-   * column of their cell; slot_first S32 [3 (Y + 1) B + 1], B = ceil((X + 1) / 16):
+  /* 2D programs, optional (fdtd_slot_order makes them): which gather slots read
+   * which part of the grid.  slot_order S32 [n <= M * 6 * K * P] lists offsets
+   * into `indices`, first the slots that are sampled (active component, nonzero
+   * mask, nonzero weight up to the point's first zero one, cell on the grid) by
+   * component, row and 16-column block of their cell; slot_first S32 [3 (Y + 1) B + 1], B = ceil((X + 1) / 16):
    * element (a (Y + 1) + j) B + b the number of them before 16-column block b of
    * row j of the a-th active component, the last one their number.
    * fdtd_launch_program advances several steps per launch only with them: each
@@ -515,6 +515,28 @@ typedef struct FdtdGatherPack {
  * columns P..Pmax-1 are left as they are (zero in a fresh plan).  No beamz
  * counterpart (its runtime packs on the host). */
 int fdtd_pack_gather(void* stream, const FdtdGatherPack* g);
+
+/* 2D gather slots sorted by the cell that they read (FdtdDft.slot_order,
+ * FdtdRecorder.order): the slots of `component_count` of the C components of a
+ * packed plan -- a program's [M, 6, K, P], or one value set's [1, 1, 1, V]. */
+typedef struct FdtdSlotOrder {
+  FdtdBuffer indices;      /* S32 [M, C, K, P] */
+  FdtdBuffer weights;      /* F32 [M, C, K, P] */
+  FdtdBuffer masks;        /* F32 [M, C], or null */
+  int32_t component_count; /* 1..3 */
+  int32_t components[3];   /* which of the C, ascending */
+  int32_t widths[3];       /* their extents along x */
+  int32_t heights[3];      /* and y */
+  int32_t rows, cols;      /* the lattice: Y + 1, X + 1 */
+  FdtdBuffer order;        /* S32 [M * component_count * K * P] */
+  FdtdBuffer first;        /* S32 [component_count * rows * ceil(cols / 16) + 1] */
+} FdtdSlotOrder;
+
+/* order: offsets into `indices`, the sampled slots (nonzero mask, nonzero weights
+ * up to this one, a cell of the component) by component, row and 16-column block
+ * of their cell, then the others; first: the number of slots before each block,
+ * the last element the number of sampled ones.  No beamz counterpart. */
+int fdtd_slot_order(void* stream, const FdtdSlotOrder* g);
 
 /* counts[v] = number of voxels with id v (U8 voxels, S32 [256] counts, set
  * to zero first): the materials a program uses, for the codebook's compact
