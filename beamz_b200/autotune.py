@@ -48,11 +48,13 @@ def heuristic(spec) -> tuple[int, int]:
     """Rules from B200 sweeps of the class step (us per step, best first):
     8-row tiles throughout; 16-plane chunks once the grid holds enough CTAs
     for many waves (512x512x256: 911 vs 952 with 8), 12-plane chunks from 7 M
-    cells (192^3: 240 vs 248 with 8 and 247 with 16, 384x300x256: 428 vs 443 and
-    441, 277x203x150: 269 vs 274), 8-plane chunks below that (192x160x96: 123
-    vs 131 with 4 and 138 with 12), 4-plane chunks for grids of up to 2.5
-    million cells, whose CTAs would otherwise not fill the GPU (128^3: 81 vs 86
-    with 8)."""
+    cells (192^3: 228 vs 233 with 8, 256x256x112: 155 vs 162), 8-plane chunks below
+    that (172x160x96: 122 vs 129 with 4, 160x168x128: 153 vs 165), 4-plane chunks
+    for grids of up to 2.5 million cells, whose CTAs would otherwise not fill the
+    GPU (128^3: 81 vs 86 with 8).  Over eleven grids of 2.6 to 13 million cells the
+    rule gains 3.8 % on dielectric, 1.5 % on conductive, 3.1 % on rectilinear and
+    3.6 % on per-site programs against the next smaller chunk; it loses 1 to 3 % on
+    128x160x128 and 384x256x128, whose CTAs then leave a short last wave."""
     cells = int(np.prod(spec.grid_shape))
     if cells >= 32 * 1024 * 1024:
         return (8, 16)

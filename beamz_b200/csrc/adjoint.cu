@@ -33,7 +33,7 @@
 // each writing only its own sites, and each set of memories is updated when its
 // last reader is done (psi_E by the E pass, psi_H by the third kernel, over the
 // absorber slabs alone).  With scratch and one launch per component and pass, a
-// 256 x 256 x 128 step moved 1.7 GB in twelve launches; this form 0.7 GB.  The
+// 256 x 256 x 128 step moved 1.7 GB in twelve launches; these two passes 0.86 GB.  The
 // permittivity gradient accumulates mu * curl'_n per E site over a design box,
 // mu = the masked E adjoint and curl'_n the forward curl.
 

@@ -884,10 +884,11 @@ cudaError_t launch_s(cudaStream_t s, const Block2D& q, int ctas, size_t smem) {
 int launch_threads(const Geo2D& g, int sms) { return g.gx * g.gy <= sms && g.rows > 512 / kGroups ? 768 : 512; }
 
 // Grids of one wave have an SM to themselves per tile: the steps are then bound
-// by a tile's own instruction chain, and 110 (80) registers a thread shorten it;
-// larger grids run two tiles per SM (us per step, 512 threads two per SM / 512
-// one per SM / 768: 400 x 400 TM 4.67 / 3.90 / 3.66, 200 x 200 3.39 / 2.88 / 3.13,
-// 1000 x 1000 12.4 / 12.6 / 14.1, 3000 x 3000 71 / 90 / 90).
+// by a tile's own instruction chain, and up to 128 (80) registers a thread shorten
+// it; larger grids run two tiles per SM (us per step with one line monitor, 512
+// threads two per SM / 512 one per SM / 768: 200 x 200 TM 3.81 / 3.29 / 3.58,
+// 400 x 400 5.13 / 4.34 / 4.08, 83 x 117 TE 3.88 / 3.36 / 3.56, 1000 x 1000 12.4 /
+// 11.8 / 13.0, 3000 x 3000 67 / 81 / 84).
 template <int Pol, bool Cpml, bool Site, bool Metric>
 cudaError_t launch_t(cudaStream_t s, const Block2D& q, int sms, int ctas, size_t smem) {
   if (q.g.gx * q.g.gy > sms) return launch_s<Pol, Cpml, Site, Metric, 512, 2>(s, q, ctas, smem);

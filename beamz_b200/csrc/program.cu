@@ -551,9 +551,10 @@ cudaError_t enqueue_sources(cudaStream_t s, const FdtdProgram& p, const Layout& 
 }
 
 // Steps per launch of 2D programs (block2d.cu).  Measured on B200, us per step
-// at 4 / 6 / 8: 400 x 400 TM 5.2 / 4.8 / 4.7, 1000 x 1000 TM 15.0 / 13.4 / 12.4
-// (12, without monitors: 4.6 against 4.4; the halo then costs more than the
-// launches it saves).
+// at 4 / 6 / 8 with one line monitor: 400 x 400 TM 4.9 / 4.5 / 4.1, 1000 x 1000
+// 13.9 / 13.1 / 12.3, 3000 x 3000 69.9 / 66.4 / 66.4 (12, which only programs
+// without monitors can take: 1000 x 1000 13.5 against 10.7; the halo then costs
+// more than the launches it saves).
 constexpr int kStepsPerLaunch2D = 8;
 
 DftDev make_dft(const FdtdProgram& p, const FdtdBuffer* bank_fields) {

@@ -87,12 +87,16 @@ def estimate_bytes(spec: ProgramSpec, schedule: str = "fused") -> int:
     by_slot = spec.ndim == 2 and slot_samples_fit(len(plans), most[1], most[0])
     for m, (points, slots) in zip(spec.monitors, plans):
         per = slots if by_slot else 1
+        dft += 12 * slots * points if by_slot else 0  # the slots by cell
         dft += 6 * len(m.freqs) * points * 8 * 2 + 6 * points * 8 * 8 + 16 * 6 * points * 4 * per
+    if spec.ndim == 2:  # the first slot of every 16 columns, of monitors and of listed recorder values
+        tables = (3 if by_slot and plans else 0) + sum(len(r.components) for r in spec.recorders if r.indices is not None)
+        dft += tables * (spec.grid_shape[0] + 1) * (spec.grid_shape[1] // 16 + 1) * 4
     records = 0
     for r in spec.recorders:
         for q, c in enumerate(r.components):
             values = int(np.prod(shapes[c])) if r.indices is None else int(np.asarray(r.indices[q]).shape[0])
-            plan = 0 if r.indices is None else values * np.asarray(r.indices[q]).shape[1] * 8
+            plan = 0 if r.indices is None else values * (np.asarray(r.indices[q]).shape[1] * 8 + 4)
             records += int(r.capacity) * values * 4 + plan
         records += int(r.capacity) * 8 + 8
     return banks * field_bytes + material + psi + dft + records + 4 * max(int(spec.total_steps), 1) + (1 << 20)
