@@ -348,6 +348,8 @@ def eps_to_coefficients_2d(eps_voxels, dt, eps0):
     """TM Ez coefficient c = dt / (eps0 eps_site), the site taking its owning
     voxel (beamz/lattice.py:935-972), as differentiable torch ops."""
     torch = _torch()
+    if eps_voxels.dim() != 2:
+        raise ValueError("eps_to_coefficients_2d takes a (ny, nx) permittivity")
     # The last voxel row and column also own the sites beyond them.
     site = torch.cat([eps_voxels, eps_voxels[-1:]], dim=0)
     site = torch.cat([site, site[:, -1:]], dim=1)
@@ -360,6 +362,8 @@ def eps_to_coefficients_3d(eps_voxels, dt, eps0):
     of the four voxels sharing each edge with clipped indices
     (beamz/lattice.py:732-786), c = fl(dt)/fl(eps0) * (1/eps_site)."""
     torch = _torch()
+    if eps_voxels.dim() != 3:
+        raise ValueError("eps_to_coefficients_3d takes a (nz, ny, nx) permittivity")
     dev = eps_voxels.device
 
     def pair(v, dim):  # the mean of each site's lower and upper voxel, clipped at the faces
