@@ -94,9 +94,9 @@ bool slot_order_ok(const FdtdProgram& p, const Layout& L, const FdtdBuffer& orde
                    int64_t most) {
   if (order.data == nullptr && first.data == nullptr) return true;
   if (p.ndim != 2 || order.data == nullptr || first.data == nullptr) return false;
-  const int64_t blocks = (L.X + kSlotBlock) / kSlotBlock;  // of X + 1 columns
-  return order.element_type == FDTD_S32 && first.element_type == FDTD_S32 && elements(order) >= 0 &&
-         elements(order) <= most && elements(first) == comps * (L.Y + 1) * blocks + 1;
+  const int64_t entries = static_cast<int64_t>(comps) * (L.Y + 1) * ((L.X + kSlotBlock) / kSlotBlock) + 1;
+  return entries < (int64_t{1} << 31) && order.element_type == FDTD_S32 && first.element_type == FDTD_S32 &&
+         elements(order) >= 0 && elements(order) <= most && elements(first) == entries;
 }
 
 int validate(const FdtdProgram& p) {

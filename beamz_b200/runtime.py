@@ -430,7 +430,7 @@ def slot_samples_fit(monitors: int, slots: int, points: int, batch: int = 16) ->
     [batch, M, 6, K, P], for several steps per launch)?  Up to 1 GiB with one slot
     per point, as many bytes as the interpolated samples take; with more slots up
     to 128 MiB, about the L2: a whole-plane monitor of four slots per point takes
-    10.8 us per step against 19 in single steps at 200 x 200 (61 MB), but 25.3
+    11 us per step against 19 in single steps at 200 x 200 (61 MB), but 25.3
     against 23.9 at 400 x 400 (245 MB)."""
     return batch >= 2 and 4 * batch * monitors * 6 * slots * points <= (1 << 30 if slots == 1 else 1 << 27)
 
@@ -749,7 +749,8 @@ class DeviceProgram:
                 setattr(s.dft, name, buf(getattr(a, name)))
             K, P = (int(v) for v in a.indices.shape[2:])
             self.slot_samples = (spec.ndim == 2 and schedule == "fused" and a.indices.numel() > 0
-                                 and slot_samples_fit(len(spec.monitors), K, P, self.dft_batch))
+                                 and slot_samples_fit(len(spec.monitors), K, P, self.dft_batch)
+                                 and 3 * lattice[0] * -(-lattice[1] // 16) < 2**31 - 1)
             if self.slot_samples:
                 comps = [COMPONENT_INDEX[c] for c in self.active]
                 order, first = _slots_by_cell(self.lib, stream, a.indices, a.weights, a.masks, comps,
